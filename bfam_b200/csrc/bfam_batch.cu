@@ -11,6 +11,7 @@
 // CUDA graph and replayed.
 #include "bfam_gpu.h"
 #include "dg_extras.cuh"
+#include "dg_mma.cuh"
 #include "dg_pglue.cuh"
 #include "dg_stage.cuh"
 #include "gpu_internal.h"
@@ -109,6 +110,48 @@ struct TileImpl
   }
 };
 
+// the matrix-instruction kernel (plain form, 3D orders 6 and 7) with a register
+// budget for MINB resident CTAs per SM
+template <int N, int MINB> struct MmaTile
+{
+  using M = MmaShape<N>;
+  static constexpr auto kernel = dg_mma_batch_kernel<N, MINB>;
+  static void launch(const DomainView *v, const int2 *w, int nwork,
+                     const StageParams &sp, const double *hops, int grid,
+                     cudaStream_t st)
+  {
+    kernel<<<grid, M::NT, M::BYTES, st>>>(v, w, nwork, sp,
+                                          1.0 / hops[7 * (N + 1) * (N + 1)]);
+  }
+  static cudaError_t prepare()
+  {
+    return cudaFuncSetAttribute((const void *)kernel,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)M::BYTES);
+  }
+  static int occupancy()
+  {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, M::NT,
+                                                      M::BYTES) != cudaSuccess)
+    {
+      cudaGetLastError();
+      return 0;
+    }
+    return n;
+  }
+  static BatchTile make()
+  {
+    BatchTile t;
+    t.NT = M::NT;
+    t.MINB = MINB;
+    t.launch = t.launch_nc = launch;
+    t.prepare = prepare;
+    t.occupancy = occupancy;
+    return t;
+  }
+};
+
 // Tile shapes per order.  Tile 0 is the single-domain kernel's shape (its
 // register budget sized for the CTAs the shared memory admits); the others
 // trade registers for resident CTAs or threads for nodes per thread (N = 7:
@@ -126,6 +169,16 @@ template <typename CT> std::vector<BatchTile> tiles_for(int dim, int N)
     // beside one element per CTA: E elements per CTA of E x threads (each
     // element its own tile and barrier), down to one warp per element at
     // the low orders (register budget for the CTAs the shared memory admits)
+    if constexpr (!use_mma<3, 7, CT>())
+    {
+      if (N == 6)
+        T0(3, 6);
+      if (N == 7)
+      {
+        T0(3, 7);
+        T(3, 7, 384, 1);
+      }
+    }
     switch (N)
     {
     case 1: T0(3, 1); TE(3, 1, 32, 8, 4); TE(3, 1, 32, 4, 8); break;
@@ -139,8 +192,6 @@ template <typename CT> std::vector<BatchTile> tiles_for(int dim, int N)
     case 5: T0(3, 5); T(3, 5, 224, 4); T(3, 5, 224, 3); T(3, 5, 224, 1);
       T(3, 5, 256, 2); TE(3, 5, 224, 2, 2);
       break;
-    case 6: T0(3, 6); break;
-    case 7: T0(3, 7); T(3, 7, 384, 1); break;
     default: break;
     }
   }
@@ -165,10 +216,31 @@ template <typename CT> std::vector<BatchTile> tiles_for(int dim, int N)
   return v;
 }
 
+// the plain form's tiles at 3D orders 6 and 7, as many as the precision form
+// has: one kernel, at N = 7 also under a register budget for one CTA
+std::vector<BatchTile> mma_tiles(int N)
+{
+  if (N == 6)
+    return {MmaTile<6, MmaShape<6>::MINB>::make()};
+  return {MmaTile<7, MmaShape<7>::MINB>::make(), MmaTile<7, 1>::make()};
+}
+
 std::vector<BatchTile> tiles(int dim, int N, int precision)
 {
+  if (dim == 3 && (N == 6 || N == 7) && precision != BFAM_GPU_PRECISION_FP32)
+    return mma_tiles(N);
   return precision == BFAM_GPU_PRECISION_FP32 ? tiles_for<float>(dim, N)
                                               : tiles_for<double>(dim, N);
+}
+
+// The table that describes an order's tiles to callers: the plain form's, and
+// at 3D orders 6 and 7, where the plain form's tiles are the matrix
+// kernel's, the precision form's (one thread per face node at least).
+std::vector<BatchTile> shape_table(int dim, int N)
+{
+  return dim == 3 && (N == 6 || N == 7)
+             ? tiles(dim, N, BFAM_GPU_PRECISION_FP32)
+             : tiles(dim, N, BFAM_GPU_PRECISION_FP64);
 }
 
 // ----------------------------------------------------- point location
@@ -746,12 +818,12 @@ int bfam_gpu_domain_get_seismograms(bfam_gpu_domain_t *d, double *out,
 
 int bfam_gpu_tile_count(int dim, int N)
 {
-  return (int)tiles(dim, N, BFAM_GPU_PRECISION_FP64).size();
+  return (int)shape_table(dim, N).size();
 }
 
 int bfam_gpu_tile_shape(int dim, int N, int tile, int *threads, int *min_ctas)
 {
-  const auto t = tiles(dim, N, BFAM_GPU_PRECISION_FP64);
+  const auto t = shape_table(dim, N);
   if (tile < 0 || tile >= (int)t.size() || !threads || !min_ctas)
     return fail(BFAM_GPU_EINVAL, "no tile %d for dim %d order %d", tile, dim,
                 N);
@@ -762,7 +834,7 @@ int bfam_gpu_tile_shape(int dim, int N, int tile, int *threads, int *min_ctas)
 
 int bfam_gpu_tile_elements(int dim, int N, int tile)
 {
-  const auto t = tiles(dim, N, BFAM_GPU_PRECISION_FP64);
+  const auto t = shape_table(dim, N);
   if (tile < 0 || tile >= (int)t.size())
     return fail(BFAM_GPU_EINVAL, "no tile %d for dim %d order %d", tile, dim,
                 N);

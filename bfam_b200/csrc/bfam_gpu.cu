@@ -7,6 +7,7 @@
 #include "bfam_gpu.h"
 #include "dg_energy.cuh"
 #include "dg_geometry.cuh"
+#include "dg_mma.cuh"
 #include "dg_stage.cuh"
 #include "gpu_internal.h"
 
@@ -55,23 +56,38 @@ constexpr auto single_kernel =
     dg_stage_kernel<DIM, N, Shape<DIM, N>::NT, stage_min_ctas<DIM, N, CT>(),
                     MODE, CT, nbuf<DIM, N, CT>()>;
 
+template <int N, int MODE>
+constexpr auto mma_kernel = dg_mma_kernel<N, MmaShape<N>::MINB, MODE>;
+
 // n work items on a persistent grid of `grid` CTAs
 template <int DIM, int N, typename CT>
 void stage_launch(const DomainView &v, int n, const StageParams &sp,
                   const double *hops, int mode, int grid, cudaStream_t stream)
 {
-  using S = Shape<DIM, N>;
-  const DiffOp<N, CT> dop = make_diffop<N, CT>(hops);
-  const size_t smem = stage_smem_bytes<DIM, N, CT>();
-  if (mode == MODE_STAGE)
-    single_kernel<DIM, N, CT, MODE_STAGE><<<grid, S::NT, smem, stream>>>(
-        v, n, sp, dop);
-  else if (mode == MODE_STAGE_NC)
-    single_kernel<DIM, N, CT, MODE_STAGE_NC><<<grid, S::NT, smem, stream>>>(
-        v, n, sp, dop);
+  if constexpr (use_mma<DIM, N, CT>())
+  {
+    using M = MmaShape<N>;
+    const double iwend = 1.0 / hops[7 * (N + 1) * (N + 1)];
+    if (mode == MODE_RHS)
+      mma_kernel<N, MODE_RHS><<<grid, M::NT, M::BYTES, stream>>>(v, n, sp, iwend);
+    else
+      mma_kernel<N, MODE_STAGE><<<grid, M::NT, M::BYTES, stream>>>(v, n, sp, iwend);
+  }
   else
-    single_kernel<DIM, N, CT, MODE_RHS><<<grid, S::NT, smem, stream>>>(
-        v, n, sp, dop);
+  {
+    using S = Shape<DIM, N>;
+    const DiffOp<N, CT> dop = make_diffop<N, CT>(hops);
+    const size_t smem = stage_smem_bytes<DIM, N, CT>();
+    if (mode == MODE_STAGE)
+      single_kernel<DIM, N, CT, MODE_STAGE><<<grid, S::NT, smem, stream>>>(
+          v, n, sp, dop);
+    else if (mode == MODE_STAGE_NC)
+      single_kernel<DIM, N, CT, MODE_STAGE_NC><<<grid, S::NT, smem, stream>>>(
+          v, n, sp, dop);
+    else
+      single_kernel<DIM, N, CT, MODE_RHS><<<grid, S::NT, smem, stream>>>(
+          v, n, sp, dop);
+  }
 }
 
 template <typename K> cudaError_t allow_smem(K kernel, int bytes)
@@ -81,23 +97,40 @@ template <typename K> cudaError_t allow_smem(K kernel, int bytes)
                               bytes);
 }
 
+template <typename K>
+cudaError_t occupancy(K kernel, int threads, size_t smem, int *occ)
+{
+  const cudaError_t e = allow_smem(kernel, (int)smem);
+  return e != cudaSuccess ? e
+                          : cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                                occ, kernel, threads, smem);
+}
+
 // shared-memory opt-in, and the resident CTAs per SM of both modes
 template <int DIM, int N, typename CT> cudaError_t stage_prepare(int *occ)
 {
-  using S = Shape<DIM, N>;
-  const int smem = (int)stage_smem_bytes<DIM, N, CT>();
-  cudaError_t e = allow_smem(single_kernel<DIM, N, CT, MODE_STAGE>, smem);
-  if (e == cudaSuccess)
-    e = allow_smem(single_kernel<DIM, N, CT, MODE_RHS>, smem);
-  if (e == cudaSuccess)
-    e = allow_smem(single_kernel<DIM, N, CT, MODE_STAGE_NC>, smem);
-  if (e == cudaSuccess)
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &occ[MODE_STAGE], single_kernel<DIM, N, CT, MODE_STAGE>, S::NT, smem);
-  if (e == cudaSuccess)
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &occ[MODE_RHS], single_kernel<DIM, N, CT, MODE_RHS>, S::NT, smem);
-  return e;
+  if constexpr (use_mma<DIM, N, CT>())
+  {
+    using M = MmaShape<N>;
+    const cudaError_t e = occupancy(mma_kernel<N, MODE_STAGE>, M::NT, M::BYTES,
+                                    &occ[MODE_STAGE]);
+    return e != cudaSuccess ? e
+                            : occupancy(mma_kernel<N, MODE_RHS>, M::NT,
+                                        M::BYTES, &occ[MODE_RHS]);
+  }
+  else
+  {
+    using S = Shape<DIM, N>;
+    const size_t smem = stage_smem_bytes<DIM, N, CT>();
+    cudaError_t e = allow_smem(single_kernel<DIM, N, CT, MODE_STAGE_NC>, (int)smem);
+    if (e == cudaSuccess)
+      e = occupancy(single_kernel<DIM, N, CT, MODE_STAGE>, S::NT, smem,
+                    &occ[MODE_STAGE]);
+    if (e == cudaSuccess)
+      e = occupancy(single_kernel<DIM, N, CT, MODE_RHS>, S::NT, smem,
+                    &occ[MODE_RHS]);
+    return e;
+  }
 }
 
 template <int DIM, int N, typename CT> KernelSet make_set()
@@ -108,8 +141,7 @@ template <int DIM, int N, typename CT> KernelSet make_set()
   k.prepare = stage_prepare<DIM, N, CT>;
   k.energy = dg_energy_kernel<DIM, N>;
   k.NT = S::NT;
-  k.smem = stage_smem_bytes<DIM, N, CT>();
-  k.nbuf = nbuf<DIM, N, CT>();
+  k.nbuf = use_mma<DIM, N, CT>() ? 1 : nbuf<DIM, N, CT>();
   return k;
 }
 

@@ -228,6 +228,12 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void *src, uint32_t bytes
                : "memory");
 }
 
+// prefetch of the line holding p into L2 (no completion)
+__device__ __forceinline__ void prefetch_l2(const void *p)
+{
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+
 // 8-byte asynchronous gather global -> shared (completes with the group)
 __device__ __forceinline__ void cp_async8(void *dst, const void *src)
 {

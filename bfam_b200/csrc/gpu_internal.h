@@ -42,7 +42,6 @@ struct KernelSet
   prepare_fn prepare = nullptr;
   energy_fn energy = nullptr;
   int NT = 0;
-  size_t smem = 0;
   int occ[2] = {0, 0}; // resident CTAs per SM of the stage and rhs kernels
   int nbuf = 1;        // element buffers per CTA
 };

@@ -428,7 +428,9 @@ int bfam_gpu_batch_add_pglue(bfam_gpu_batch_t *b, bfam_gpu_pglue_t *g);
  * than nodes or face nodes loops over them; each element of a CTA has its
  * own shared-memory tile and barrier, down to one warp per element) and a
  * register budget for `min_ctas` resident CTAs per SM.  Tile 0 is the
- * single-domain kernel's (one element per CTA). */
+ * single-domain kernel's (one element per CTA).  At 3D orders 6 and 7 the
+ * shapes are the precision form's; the plain form's tiles there are one warp
+ * per plane of nodes. */
 int bfam_gpu_tile_count(int dim, int N);
 int bfam_gpu_tile_shape(int dim, int N, int tile, int *threads,
                         int *min_ctas);
