@@ -31,9 +31,9 @@ namespace
 
 // ------------------------------------------------------------ batch tiles
 
-typedef void (*batch_launch_fn)(const DomainView *, const int2 *, int,
+typedef cudaError_t (*batch_launch_fn)(const DomainView *, const int2 *, int,
                                 const StageParams &, const double *hops,
-                                int grid, cudaStream_t);
+                                int grid, cudaStream_t, bool overlap);
 typedef cudaError_t (*batch_prepare_fn)();
 typedef int (*batch_occupancy_fn)();
 
@@ -59,19 +59,21 @@ struct TileImpl
   static constexpr auto kernel_nc =
       dg_stage_batch_kernel<DIM, N, NT, MINB, MODE_STAGE_NC, CT, NB, EPC>;
   static constexpr size_t SMEM = stage_smem_bytes<DIM, N, CT, EPC>();
-  static void launch(const DomainView *v, const int2 *w, int nwork,
+  static cudaError_t launch(const DomainView *v, const int2 *w, int nwork,
                      const StageParams &sp, const double *hops, int grid,
-                     cudaStream_t st)
+                     cudaStream_t st, bool overlap)
   {
     const DiffOp<N, CT> dop = make_diffop<N, CT>(hops);
-    kernel<<<grid, NT * EPC, SMEM, st>>>(v, w, nwork, sp, dop);
+    return launch_dependent(overlap, kernel, grid, NT * EPC, SMEM, st, v, w, nwork, sp,
+                            dop);
   }
-  static void launch_nc(const DomainView *v, const int2 *w, int nwork,
+  static cudaError_t launch_nc(const DomainView *v, const int2 *w, int nwork,
                         const StageParams &sp, const double *hops, int grid,
-                        cudaStream_t st)
+                        cudaStream_t st, bool overlap)
   {
     const DiffOp<N, CT> dop = make_diffop<N, CT>(hops);
-    kernel_nc<<<grid, NT * EPC, SMEM, st>>>(v, w, nwork, sp, dop);
+    return launch_dependent(overlap, kernel_nc, grid, NT * EPC, SMEM, st, v, w, nwork,
+                            sp, dop);
   }
   static cudaError_t prepare()
   {
@@ -116,12 +118,12 @@ template <int N, int MINB> struct MmaTile
 {
   using M = MmaShape<N>;
   static constexpr auto kernel = dg_mma_batch_kernel<N, MINB>;
-  static void launch(const DomainView *v, const int2 *w, int nwork,
+  static cudaError_t launch(const DomainView *v, const int2 *w, int nwork,
                      const StageParams &sp, const double *hops, int grid,
-                     cudaStream_t st)
+                     cudaStream_t st, bool overlap)
   {
-    kernel<<<grid, M::NT, M::BYTES, st>>>(v, w, nwork, sp,
-                                          1.0 / hops[7 * (N + 1) * (N + 1)]);
+    return launch_dependent(overlap, kernel, grid, M::NT, M::BYTES, st, v, w, nwork, sp,
+                            1.0 / hops[7 * (N + 1) * (N + 1)]);
   }
   static cudaError_t prepare()
   {
@@ -301,6 +303,12 @@ void node_weights(const bfam_gpu_domain_t *d, const double *xi, double *wn)
   }
 }
 
+// receiver CTAs per domain of the post-step kernel
+unsigned post_parts(int nrecv)
+{
+  return (unsigned)std::min(std::max(nrecv, 1), POST_PARTS);
+}
+
 PostView post_view(bfam_gpu_domain_t *d, int cur, double dt)
 {
   PostView p;
@@ -336,9 +344,10 @@ int set_clock(bfam_gpu_domain_t *d, double t, int reset)
 
 int launch_post(bfam_gpu_domain_t *d, int cur, double dt)
 {
-  dg_post_step_one<<<1, POST_THREADS, 0, d->stream>>>(post_view(d, cur, dt));
+  CUDA_TRY(launch_dependent(true, dg_post_step_one, dim3(1, post_parts(d->nrecv)),
+                            POST_THREADS, 0, d->stream,
+                            post_view(d, cur, dt)));
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  CUDA_TRY(cudaGetLastError());
   return 0;
 }
 
@@ -356,6 +365,7 @@ struct bfam_gpu_batch
     std::vector<double> hops;
     std::vector<BatchTile> tiles;
     int tile = 0, ctas_per_sm = 0;
+    int multi_tile = 0; // default tile of a group of several domains
     int64_t nwork = 0; // elements of all levels
     DomainView *views[2] = {nullptr, nullptr}; // per batch parity
     // per launch level: (domain, element) work list, its length and grid
@@ -526,6 +536,45 @@ int upload_views(bfam_gpu_batch_t *b)
   return 0;
 }
 
+// the post-step kernel over all domains
+cudaError_t launch_post_step(bfam_gpu_batch_t *b, int p)
+{
+  int nrecv = 0;
+  for (const auto *d : b->doms)
+    nrecv = std::max(nrecv, d->nrecv);
+  return launch_dependent(true, dg_post_step_kernel,
+                          dim3((unsigned)b->doms.size(), post_parts(nrecv)),
+                          POST_THREADS, 0, b->stream, b->post[p]);
+}
+
+// Level l of group g's stage sp, from state parity par.  A group of one domain
+// under the default tile runs the single-domain kernel (the same arithmetic
+// with the domain's view in the parameter bank: at N = 5 in FP64 the batch
+// kernel, which reads its view from memory, spills at five CTAs per SM).
+int launch_level(bfam_gpu_batch_t *b, bfam_gpu_batch::Group &g, size_t l,
+                 int par, const StageParams &sp, cudaStream_t st, bool overlap)
+{
+  const bool nc = l == 0 && g.level0_nc;
+  if (g.doms.size() == 1 && g.tile == 0 && g.ctas_per_sm == 0)
+  {
+    const int i = g.doms[0];
+    bfam_gpu_domain_t *d = b->doms[i];
+    DomainView v = view(d, (b->cur0[i] + par) & 1);
+    v.dt = b->dt[i];
+    if (d->nlevels > 1)
+      v.elist = d->elist + d->level_off[l];
+    CUDA_TRY(d->ks.launch(v, (int)g.nwork_l[l], sp, g.hops.data(),
+                          nc ? MODE_STAGE_NC : MODE_STAGE, g.grid[l], st,
+                          overlap));
+    return 0;
+  }
+  const BatchTile &t = g.tiles[g.tile];
+  CUDA_TRY((nc ? t.launch_nc : t.launch)(g.views[par], g.work[l],
+                                         (int)g.nwork_l[l], sp, g.hops.data(),
+                                         g.grid[l], st, overlap));
+  return 0;
+}
+
 // one step from batch parity p: every stage of every group, then the
 // post-step kernel over all domains
 int issue_step_glued(bfam_gpu_batch_t *b, int p);
@@ -537,8 +586,11 @@ int issue_step(bfam_gpu_batch_t *b, int p)
   int launches = 0;
   for (auto &g : b->groups)
   {
-    CUDA_TRY(cudaStreamWaitEvent(g.stream, b->fork, 0));
-    const BatchTile &t = g.tiles[g.tile];
+    // the first group stays on the batch's stream, the others fork from it
+    const bool forked = &g != &b->groups[0];
+    cudaStream_t st = forked ? g.stream : b->stream;
+    if (forked)
+      CUDA_TRY(cudaStreamWaitEvent(st, b->fork, 0));
     for (int s = 0; s < b->ns; ++s)
     {
       StageParams sp;
@@ -553,19 +605,20 @@ int issue_step(bfam_gpu_batch_t *b, int p)
       // hanging faces
       for (size_t l = 0; l < g.work.size(); ++l)
       {
-        (l == 0 && g.level0_nc ? t.launch_nc : t.launch)(
-            g.views[(p + s) & 1], g.work[l], (int)g.nwork_l[l], sp,
-            g.hops.data(), g.grid[l], g.stream);
-        CUDA_TRY(cudaGetLastError());
+        // one chain of launches overlaps them; with several groups the
+        // waiting CTAs would take the other groups' places
+        if (int rc = launch_level(b, g, l, (p + s) & 1, sp, st,
+                                  b->groups.size() == 1))
+          return rc;
         ++launches;
       }
     }
-    CUDA_TRY(cudaEventRecord(g.done, g.stream));
-    CUDA_TRY(cudaStreamWaitEvent(b->stream, g.done, 0));
+    if (forked)
+      CUDA_TRY(cudaEventRecord(g.done, st));
   }
-  dg_post_step_kernel<<<(int)b->doms.size(), POST_THREADS, 0, b->stream>>>(
-      b->post[p]);
-  CUDA_TRY(cudaGetLastError());
+  for (size_t k = 1; k < b->groups.size(); ++k)
+    CUDA_TRY(cudaStreamWaitEvent(b->stream, b->groups[k].done, 0));
+  CUDA_TRY(launch_post_step(b, p));
   ++launches;
   g_launches.fetch_add(launches, std::memory_order_relaxed);
   return 0;
@@ -618,18 +671,18 @@ int issue_step_glued(bfam_gpu_batch_t *b, int p)
     for (size_t k = 0; k < b->pglues.size(); ++k)
     {
       const PGlueView v = pglue_view(b, k, par);
-      if (b->doms[0]->dim == 3)
-        dg_pglue_kernel<3><<<v.K, PGLUE_THREADS, 0, b->stream>>>(v);
-      else
-        dg_pglue_kernel<2><<<v.K, PGLUE_THREADS, 0, b->stream>>>(v);
-      CUDA_TRY(cudaGetLastError());
+      CUDA_TRY(launch_dependent(false, b->doms[0]->dim == 3 ? dg_pglue_kernel<3>
+                                                     : dg_pglue_kernel<2>,
+                                v.K, PGLUE_THREADS, 0, b->stream, v));
       ++launches;
     }
     CUDA_TRY(cudaEventRecord(b->fork, b->stream));
     for (auto &g : b->groups)
     {
-      CUDA_TRY(cudaStreamWaitEvent(g.stream, b->fork, 0));
-      const BatchTile &t = g.tiles[g.tile];
+      const bool forked = &g != &b->groups[0];
+      cudaStream_t st = forked ? g.stream : b->stream;
+      if (forked)
+        CUDA_TRY(cudaStreamWaitEvent(st, b->fork, 0));
       StageParams sp;
       sp.A = b->A[s];
       sp.B = b->B[s];
@@ -640,19 +693,17 @@ int issue_step_glued(bfam_gpu_batch_t *b, int p)
       sp.ahead = g.ahead;
       for (size_t l = 0; l < g.work.size(); ++l)
       {
-        (l == 0 && g.level0_nc ? t.launch_nc : t.launch)(
-            g.views[par], g.work[l], (int)g.nwork_l[l], sp, g.hops.data(),
-            g.grid[l], g.stream);
-        CUDA_TRY(cudaGetLastError());
+        if (int rc = launch_level(b, g, l, par, sp, st, false))
+          return rc;
         ++launches;
       }
-      CUDA_TRY(cudaEventRecord(g.done, g.stream));
-      CUDA_TRY(cudaStreamWaitEvent(b->stream, g.done, 0));
+      if (forked)
+        CUDA_TRY(cudaEventRecord(g.done, st));
     }
+    for (size_t k = 1; k < b->groups.size(); ++k)
+      CUDA_TRY(cudaStreamWaitEvent(b->stream, b->groups[k].done, 0));
   }
-  dg_post_step_kernel<<<(int)b->doms.size(), POST_THREADS, 0, b->stream>>>(
-      b->post[p]);
-  CUDA_TRY(cudaGetLastError());
+  CUDA_TRY(launch_post_step(b, p));
   ++launches;
   g_launches.fetch_add(launches, std::memory_order_relaxed);
   return 0;
@@ -926,6 +977,10 @@ int bfam_gpu_batch_create(bfam_gpu_domain_t *const *doms, int ndom,
       G.flux = d->flux;
       G.hops = d->hops;
       G.tiles = tiles(d->dim, d->N, d->precision);
+      // several domains at N = 5 in FP64: the four-CTA tile, whose batch
+      // kernel does not spill (104 against 100 G DOF-updates/s)
+      G.multi_tile = d->dim == 3 && d->N == 5 &&
+                     d->precision == BFAM_GPU_PRECISION_FP64;
       if (G.tiles.empty())
       {
         batch_release(b);
@@ -940,6 +995,8 @@ int bfam_gpu_batch_create(bfam_gpu_domain_t *const *doms, int ndom,
   }
   for (auto &G : b->groups)
   {
+    if (G.doms.size() > 1)
+      G.tile = G.multi_tile;
     if (G.nwork > INT32_MAX)
     {
       batch_release(b);

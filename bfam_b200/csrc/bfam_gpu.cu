@@ -61,32 +61,30 @@ constexpr auto mma_kernel = dg_mma_kernel<N, MmaShape<N>::MINB, MODE>;
 
 // n work items on a persistent grid of `grid` CTAs
 template <int DIM, int N, typename CT>
-void stage_launch(const DomainView &v, int n, const StageParams &sp,
-                  const double *hops, int mode, int grid, cudaStream_t stream)
+cudaError_t stage_launch(const DomainView &v, int n, const StageParams &sp,
+                         const double *hops, int mode, int grid,
+                         cudaStream_t stream, bool overlap)
 {
   if constexpr (use_mma<DIM, N, CT>())
   {
     using M = MmaShape<N>;
     const double iwend = 1.0 / hops[7 * (N + 1) * (N + 1)];
-    if (mode == MODE_RHS)
-      mma_kernel<N, MODE_RHS><<<grid, M::NT, M::BYTES, stream>>>(v, n, sp, iwend);
-    else
-      mma_kernel<N, MODE_STAGE><<<grid, M::NT, M::BYTES, stream>>>(v, n, sp, iwend);
+    return launch_dependent(overlap,
+                            mode == MODE_RHS ? mma_kernel<N, MODE_RHS>
+                                             : mma_kernel<N, MODE_STAGE>,
+                            grid, M::NT, M::BYTES, stream, v, n, sp, iwend);
   }
   else
   {
     using S = Shape<DIM, N>;
     const DiffOp<N, CT> dop = make_diffop<N, CT>(hops);
     const size_t smem = stage_smem_bytes<DIM, N, CT>();
-    if (mode == MODE_STAGE)
-      single_kernel<DIM, N, CT, MODE_STAGE><<<grid, S::NT, smem, stream>>>(
-          v, n, sp, dop);
-    else if (mode == MODE_STAGE_NC)
-      single_kernel<DIM, N, CT, MODE_STAGE_NC><<<grid, S::NT, smem, stream>>>(
-          v, n, sp, dop);
-    else
-      single_kernel<DIM, N, CT, MODE_RHS><<<grid, S::NT, smem, stream>>>(
-          v, n, sp, dop);
+    return launch_dependent(
+        overlap,
+        mode == MODE_STAGE      ? single_kernel<DIM, N, CT, MODE_STAGE>
+        : mode == MODE_STAGE_NC ? single_kernel<DIM, N, CT, MODE_STAGE_NC>
+                                : single_kernel<DIM, N, CT, MODE_RHS>,
+        grid, S::NT, smem, stream, v, n, sp, dop);
   }
 }
 
@@ -426,9 +424,9 @@ int launch_stage(bfam_gpu_domain_t *d, int in, double A, double B, double C,
       pl.bytes = per_dof * (double)n * d->Np * d->NFLD;
       CUDA_TRY(cudaEventRecord(pl.t0, d->stream));
     }
-    d->ks.launch(v, n, sp, d->hops.data(), m, grid, d->stream);
+    CUDA_TRY(d->ks.launch(v, n, sp, d->hops.data(), m, grid, d->stream,
+                           true));
     g_launches.fetch_add(1, std::memory_order_relaxed);
-    CUDA_TRY(cudaGetLastError());
     if (d->prof)
     {
       CUDA_TRY(cudaEventRecord(pl.t1, d->stream));

@@ -37,7 +37,7 @@ struct DomainClock
 {
   double time; // time at the start of the current step
   int nsamp;   // receiver samples recorded
-  int pad;
+  int ticket;  // finished CTAs of the post-step kernel, zero between steps
 };
 
 // Ricker point force of a domain (src_elem < 0: none).  Per node of the
@@ -226,6 +226,18 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void *src, uint32_t bytes
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src),
                "r"(bytes)
                : "memory");
+}
+
+// Programmatic dependent launch: let the next kernel's CTAs start (they wait
+// for this grid's completion themselves), and wait for the completion of the
+// kernel before this one.  Without the launch attribute both do nothing.
+__device__ __forceinline__ void grid_launch_dependents()
+{
+  asm volatile("griddepcontrol.launch_dependents;");
+}
+__device__ __forceinline__ void grid_dependency_wait()
+{
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // prefetch of the line holding p into L2 (no completion)

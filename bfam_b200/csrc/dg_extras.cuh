@@ -21,44 +21,70 @@ struct PostView
   double dt;
 };
 
-// One CTA per domain: sample every field at every receiver (one warp per
-// (receiver, field) pair, lane-strided dot product with the element's
-// Lagrange weights, then a butterfly sum: deterministic for a fixed block
-// size), then advance the domain's clock by dt.  Samples beyond
+// Sample every field at the receivers blockIdx.y, blockIdx.y + gridDim.y, ...
+// of one domain: one warp per (receiver, field) pair, lane-strided dot product
+// with the element's Lagrange weights, then a butterfly sum (deterministic:
+// the order does not depend on the grid).  The last of the domain's CTAs to
+// finish, by a ticket in its clock, advances the clock by dt.  Samples beyond
 // max_samples are dropped; the clock still advances.
+// What bounds it is the latency of one (receiver, field) pair, two dependent
+// trips to memory: a single CTA took them 18 deep for 16 receivers of nine
+// fields, 10 to 14 us of a step (N = 3 and 5), so a CTA of nine warps takes
+// one receiver instead.
 __device__ __forceinline__ void post_step(const PostView &p)
 {
-  const int s = p.clock->nsamp;
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const int nr = p.nrecv > 1 ? p.nrecv : 1;
+  const int parts = nr < (int)gridDim.y ? nr : (int)gridDim.y;
+  if ((int)blockIdx.y >= parts)
+    return;
+  const int s = *static_cast<volatile int *>(&p.clock->nsamp);
   if (s < p.max_samples)
   {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5,
               nw = blockDim.x >> 5;
-    for (int w = wid; w < p.nrecv * p.nfld; w += nw)
+    for (int r = blockIdx.y; r < p.nrecv; r += parts)
     {
-      const int r = w / p.nfld, c = w % p.nfld;
-      const double *x = p.q + c * p.fs + (size_t)p.relem[r] * p.Np;
+      const size_t at = (size_t)p.relem[r] * p.Np;
       const double *wt = p.rw + (size_t)r * p.Np;
-      double acc = 0;
-      for (int n = lane; n < p.Np; n += 32)
-        acc += wt[n] * x[n];
+      for (int c = wid; c < p.nfld; c += nw)
+      {
+        const double *x = p.q + c * p.fs + at;
+        double acc = 0;
+#pragma unroll 4
+        for (int n = lane; n < p.Np; n += 32)
+          acc += wt[n] * x[n];
 #pragma unroll
-      for (int o = 16; o; o >>= 1)
-        acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      if (lane == 0)
-        p.seis[((size_t)s * p.nrecv + r) * p.nfld + c] = acc;
+        for (int o = 16; o; o >>= 1)
+          acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (lane == 0)
+          p.seis[((size_t)s * p.nrecv + r) * p.nfld + c] = acc;
+      }
     }
   }
   __syncthreads(); // every warp has read the clock
   if (threadIdx.x == 0)
   {
-    p.clock->time += p.dt;
-    p.clock->nsamp = s + 1;
+    bool last = parts == 1;
+    if (!last)
+    {
+      __threadfence(); // this CTA's reads come before its ticket
+      last = atomicAdd(&p.clock->ticket, 1) == parts - 1;
+    }
+    if (last)
+    {
+      p.clock->time += p.dt;
+      p.clock->nsamp = s + 1;
+      p.clock->ticket = 0;
+    }
   }
 }
 
-constexpr int POST_THREADS = 256;
+constexpr int POST_THREADS = 288; // a warp per field
+constexpr int POST_PARTS = 64;    // receiver CTAs per domain, at most
 
-// batches: one CTA per domain of the array
+// batches: CTAs (domain, part) over the array's domains
 __global__ void __launch_bounds__(POST_THREADS)
     dg_post_step_kernel(const PostView *__restrict__ pv)
 {

@@ -210,8 +210,13 @@ __device__ __forceinline__ void mma_element(const Item &item, int n,
 
   // ------------------------------------------------------------------ issue
   if (t == 0)
-  {
     mbar_init(bar, 1);
+  int2 ds = make_int2(0, 2);
+  if (w < 6)
+    ds = d.fdesc[(size_t)e * 6 + w];
+  grid_dependency_wait(); // the stage input is complete
+  if (t == 0)
+  {
     fence_proxy_async();
     // the last row of an odd-sized state has no value after it to copy
     const bool last = Np % 2 && e == d.K - 1 && (d.K & 1);
@@ -262,11 +267,9 @@ __device__ __forceinline__ void mma_element(const Item &item, int n,
   }
   const int fo = a0 * sa + r * sb, pn = i0 + Nq * r;
   double *pj = pt + f * 6 * P + pn;
-  int2 ds = make_int2(0, 2);
   double2 nb[6];
   if (w < 6)
   {
-    ds = d.fdesc[(size_t)e * 6 + f];
     const int kind = ds.y & 3;
     if (kind < 2)
     {
@@ -477,7 +480,7 @@ __device__ __forceinline__ void mma_element(const Item &item, int n,
   const double2 fx = make_double2(dfrag(2 * c), dfrag(2 * c + 1));
   const double2 fy = YS ? make_double2(dfrag(c), dfrag(c + 4)) : fx;
   __syncthreads();
-  // ----------------------------------------------------------------- update
+  grid_launch_dependents(); // as in dg_stage.cuh, not earlier
   const double a = MODE != MODE_RHS ? sp.A : 0.0;
   const double s = MODE != MODE_RHS ? d.dt : 1.0;
   const int n0 = w * P + r * Nq + i0, m0 = n0 + w * (PP - P);

@@ -112,6 +112,8 @@ __global__ void __launch_bounds__(PGLUE_THREADS) dg_pglue_kernel(const PGlueView
   __shared__ double tmp[NTF][MF];
   __shared__ double J[2][NJ][MF];
   const int k = blockIdx.x, t = threadIdx.x;
+  grid_launch_dependents();
+  grid_dependency_wait();
   if (k >= v.K)
     return;
   const int Ngq = v.Ng + 1;

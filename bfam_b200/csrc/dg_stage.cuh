@@ -578,6 +578,11 @@ __device__ __forceinline__ void compute_element(const DomainView &d,
   }
   Sub<NT, EPC>::sync();
 
+  // The next launch may start from here (all CTAs past this point): released
+  // at the kernel's start instead, its waiting CTAs crowd onto the SMs that
+  // drain first (N = 5 on 1,057 elements 133 us per step against 127, 129
+  // without the overlap)
+  grid_launch_dependents();
   // ------------------------ phase 2: volume, face contributions and update
   constexpr bool DQS = stage_dqs<DIM, N, CT>();
   if (MODE != MODE_RHS && rd && DQS)
@@ -698,6 +703,7 @@ __device__ __forceinline__ void stage_loop(const Item &item, int n,
   }
   SB::sync();
   int idx = (int)blockIdx.x * EPC + SB::id();
+  grid_dependency_wait(); // the stage input is complete
   if (idx >= n)
     return;
   if constexpr (NBUF == 1)
