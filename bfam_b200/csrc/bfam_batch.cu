@@ -12,6 +12,7 @@
 #include "bfam_gpu.h"
 #include "dg_extras.cuh"
 #include "dg_mma.cuh"
+#include "dg_pack.cuh"
 #include "dg_pglue.cuh"
 #include "dg_stage.cuh"
 #include "gpu_internal.h"
@@ -41,6 +42,7 @@ struct BatchTile
 {
   int NT = 0, MINB = 0, NBUF = 1;
   int EPC = 1; // elements per CTA (NT threads each)
+  int pack = 0; // elements per CTA of the packed kernel (0: not packed)
   batch_launch_fn launch = nullptr;
   // the same tile compiled without the coarse-face pass, for launches
   // whose elements have no coarse-side hanging face (level 0 of domains
@@ -112,6 +114,68 @@ struct TileImpl
   }
 };
 
+// the packed kernel as the first tile of a shape that it serves; reported to
+// callers as the shape's one-element tile
+template <int DIM, int N, typename CT> struct PackTile
+{
+  using K = PackShape<DIM, N, CT>;
+  template <int MODE>
+  static cudaError_t run(const DomainView *v, const int2 *w, int nwork,
+                         const StageParams &sp, const double *hops, int,
+                         cudaStream_t st, bool overlap)
+  {
+    const DiffOp<N, CT> dop = make_diffop<N, CT>(hops);
+    return launch_dependent(overlap, dg_pack_batch_kernel<DIM, N, MODE, CT>,
+                            (nwork + K::E - 1) / K::E, K::NT, K::BYTES, st, v,
+                            w, nwork, sp, dop);
+  }
+  static cudaError_t prepare()
+  {
+    cudaError_t e = cudaFuncSetAttribute(
+        (const void *)dg_pack_batch_kernel<DIM, N, MODE_STAGE, CT>,
+        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)K::BYTES);
+    return e != cudaSuccess
+               ? e
+               : cudaFuncSetAttribute(
+                     (const void *)dg_pack_batch_kernel<DIM, N, MODE_STAGE_NC, CT>,
+                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)K::BYTES);
+  }
+  static int occupancy()
+  {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+            &n, dg_pack_batch_kernel<DIM, N, MODE_STAGE, CT>, K::NT, K::BYTES) !=
+        cudaSuccess)
+    {
+      cudaGetLastError();
+      return 0;
+    }
+    return n;
+  }
+  static BatchTile make()
+  {
+    BatchTile t;
+    t.NT = Shape<DIM, N>::NT;
+    t.MINB = stage_min_ctas<DIM, N, CT>();
+    t.pack = K::E;
+    t.launch = run<MODE_STAGE>;
+    t.launch_nc = run<MODE_STAGE_NC>;
+    t.prepare = prepare;
+    t.occupancy = occupancy;
+    return t;
+  }
+};
+
+// the first tile of a shape: the single-domain kernel's
+template <int DIM, int N, typename CT> BatchTile first_tile()
+{
+  if constexpr (use_pack<DIM, N, CT>())
+    return PackTile<DIM, N, CT>::make();
+  else
+    return TileImpl<DIM, N, Shape<DIM, N>::NT, stage_min_ctas<DIM, N, CT>(),
+                    CT>::make();
+}
+
 // the matrix-instruction kernel (plain form, 3D orders 6 and 7) with a register
 // budget for MINB resident CTAs per SM
 template <int N, int MINB> struct MmaTile
@@ -165,7 +229,7 @@ template <typename CT> std::vector<BatchTile> tiles_for(int dim, int N)
   std::vector<BatchTile> v;
 #define T(D, NN, NT, MB) v.push_back(TileImpl<D, NN, NT, MB, CT>::make())
 #define TE(D, NN, NT, MB, E) v.push_back(TileImpl<D, NN, NT, MB, CT, E>::make())
-#define T0(D, NN) T(D, NN, (Shape<D, NN>::NT), (stage_min_ctas<D, NN, CT>()))
+#define T0(D, NN) v.push_back(first_tile<D, NN, CT>())
   if (dim == 3)
   {
     // beside one element per CTA: E elements per CTA of E x threads (each
@@ -487,8 +551,9 @@ int choose_grid(bfam_gpu_batch_t *b, bfam_gpu_batch_t::Group &g)
   // one-buffer tiles
   const bool persistent = t.NBUF == 2;
   // L2 lookahead in work items: half a wave of resident elements
+  const int epc = t.pack ? t.pack : t.EPC;
   g.ahead = persistent ? 0
-                       : (int)std::min<int64_t>(full * t.EPC / 2, INT32_MAX);
+                       : (int)std::min<int64_t>(full * epc / 2, INT32_MAX);
   g.grid.resize(g.nwork_l.size());
   for (size_t l = 0; l < g.nwork_l.size(); ++l)
     g.grid[l] = (int)(persistent ? (g.nwork_l[l] > full ? full : g.nwork_l[l])

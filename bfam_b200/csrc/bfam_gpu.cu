@@ -8,6 +8,7 @@
 #include "dg_energy.cuh"
 #include "dg_geometry.cuh"
 #include "dg_mma.cuh"
+#include "dg_pack.cuh"
 #include "dg_stage.cuh"
 #include "gpu_internal.h"
 
@@ -74,6 +75,17 @@ cudaError_t stage_launch(const DomainView &v, int n, const StageParams &sp,
                                              : mma_kernel<N, MODE_STAGE>,
                             grid, M::NT, M::BYTES, stream, v, n, sp, iwend);
   }
+  else if constexpr (use_pack<DIM, N, CT>())
+  {
+    using K = PackShape<DIM, N, CT>;
+    const DiffOp<N, CT> dop = make_diffop<N, CT>(hops);
+    return launch_dependent(
+        overlap,
+        mode == MODE_STAGE      ? dg_pack_kernel<DIM, N, MODE_STAGE, CT>
+        : mode == MODE_STAGE_NC ? dg_pack_kernel<DIM, N, MODE_STAGE_NC, CT>
+                                : dg_pack_kernel<DIM, N, MODE_RHS, CT>,
+        (n + K::E - 1) / K::E, K::NT, K::BYTES, stream, v, n, sp, dop);
+  }
   else
   {
     using S = Shape<DIM, N>;
@@ -116,6 +128,19 @@ template <int DIM, int N, typename CT> cudaError_t stage_prepare(int *occ)
                             : occupancy(mma_kernel<N, MODE_RHS>, M::NT,
                                         M::BYTES, &occ[MODE_RHS]);
   }
+  else if constexpr (use_pack<DIM, N, CT>())
+  {
+    using K = PackShape<DIM, N, CT>;
+    cudaError_t e =
+        allow_smem(dg_pack_kernel<DIM, N, MODE_STAGE_NC, CT>, (int)K::BYTES);
+    if (e == cudaSuccess)
+      e = occupancy(dg_pack_kernel<DIM, N, MODE_STAGE, CT>, K::NT, K::BYTES,
+                    &occ[MODE_STAGE]);
+    if (e == cudaSuccess)
+      e = occupancy(dg_pack_kernel<DIM, N, MODE_RHS, CT>, K::NT, K::BYTES,
+                    &occ[MODE_RHS]);
+    return e;
+  }
   else
   {
     using S = Shape<DIM, N>;
@@ -139,7 +164,11 @@ template <int DIM, int N, typename CT> KernelSet make_set()
   k.prepare = stage_prepare<DIM, N, CT>;
   k.energy = dg_energy_kernel<DIM, N>;
   k.NT = S::NT;
-  k.nbuf = use_mma<DIM, N, CT>() ? 1 : nbuf<DIM, N, CT>();
+  if (use_pack<DIM, N, CT>())
+    k.elements = PackShape<DIM, N, CT>::E;
+  k.nbuf = use_mma<DIM, N, CT>() || use_pack<DIM, N, CT>()
+               ? 1
+               : nbuf<DIM, N, CT>();
   return k;
 }
 
@@ -380,7 +409,9 @@ int launch_stage(bfam_gpu_domain_t *d, int in, double A, double B, double C,
   sp.flux = d->flux;
   // one element per CTA: prefetch half a wave of resident CTAs ahead (about
   // half a CTA lifetime before the element's CTA starts)
-  sp.ahead = d->ks.nbuf == 1 ? d->ks.occ[mode] * d->sms / 2 : 0;
+  sp.ahead = d->ks.nbuf == 1
+                 ? d->ks.occ[mode] * d->sms * d->ks.elements / 2
+                 : 0;
   DomainView v = view(d, in);
   v.dt = dt;
   // one launch per level; level l's elements after level l-1's

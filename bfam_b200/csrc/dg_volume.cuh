@@ -92,14 +92,15 @@ template <int DIM, int N, typename CT> constexpr int dparam_axes()
 // contractions of src/bfam.c:3519-3624 evaluated at one node.  qs is the
 // element's state tile in CT, sD the column-major D(i,m) = sD[i + Nq m], both
 // in shared memory, dop the same operators in the kernel's parameter space.
-template <int DIM, int N, typename CT>
+// FS separates the fields in the tile.
+template <int DIM, int N, typename CT, int FS = Shape<DIM, N>::Np>
 __device__ __forceinline__ void volume_node(const CT *qs, const CT *sD,
                                             const DiffOp<N, CT> &dop,
                                             const ElemData &me, double s, int i,
                                             int j, int k, CT *rv)
 {
   using S = Shape<DIM, N>;
-  constexpr int Nq = S::Nq, Np = S::Np, NFLD = S::NFLD;
+  constexpr int Nq = S::Nq, NFLD = S::NFLD;
   const CT lam = CT(me.lam), mu = CT(me.mu), irho = CT(me.irho);
   const CT l2m = lam + CT(2) * mu;
 #pragma unroll
@@ -109,10 +110,10 @@ __device__ __forceinline__ void volume_node(const CT *qs, const CT *sD,
   // derivative of field c along axis ax at this node
   auto deriv = [&](int c, int ax, const CT *Dl) {
     if (ax == 0)
-      return line_dx<N, CT>(qs + c * Np + Nq * (j + Nq * k), Dl);
+      return line_dx<N, CT>(qs + c * FS + Nq * (j + Nq * k), Dl);
     if (ax == 1)
-      return line_ds<N, Nq, CT>(qs + c * Np + i + Nq * Nq * k, Dl);
-    return line_ds<N, Nq * Nq, CT>(qs + c * Np + i + Nq * j, Dl);
+      return line_ds<N, Nq, CT>(qs + c * FS + i + Nq * Nq * k, Dl);
+    return line_ds<N, Nq * Nq, CT>(qs + c * FS + i + Nq * j, Dl);
   };
 
   constexpr int PA = dparam_axes<DIM, N, CT>();
@@ -193,11 +194,22 @@ __device__ __forceinline__ void volume_node(const CT *qs, const CT *sD,
   }
 }
 
+__device__ __forceinline__ double fma_ct(double a, double b, double c)
+{
+  return __fma_rn(a, b, c);
+}
+__device__ __forceinline__ float fma_ct(float a, float b, float c)
+{
+  return __fmaf_rn(a, b, c);
+}
+
 // Lifted face contribution of one face point: jump terms J = (T* - T-,
 // v* - v-) times the lift factor L = s (2/h_ax) / w_0 of the lumped LGL mass,
 // mapped onto the fields (outward normal n = sg e_ax):
 //   v += L / rho (T* - T-),
 //   S += L (lambda (dv.n) I + mu (dv n^T + n dv^T)).
+// The normal stress is the sum of two products; which of them is rounded is
+// stated here, so that every kernel gives the same value.
 template <int DIM, typename CT>
 __device__ __forceinline__ void lift_face(const CT *J, int ax, CT sg, CT L,
                                           const ElemData &me, CT *out)
@@ -213,9 +225,9 @@ __device__ __forceinline__ void lift_face(const CT *J, int ax, CT sg, CT L,
     out[0] = Li * J[0];
     out[1] = Li * J[1];
     out[2] = Li * J[2];
-    out[3] = ll + (x ? two * lm * dv0 : zero);
-    out[4] = ll + (y ? two * lm * dv1 : zero);
-    out[5] = ll + (z ? two * lm * dv2 : zero);
+    out[3] = x ? fma_ct(two * lm, dv0, ll) : ll;
+    out[4] = y ? fma_ct(two * lm, dv1, ll) : ll;
+    out[5] = z ? fma_ct(two * lm, dv2, ll) : ll;
     out[6] = lm * ((y ? dv0 : zero) + (x ? dv1 : zero));
     out[7] = lm * ((z ? dv0 : zero) + (x ? dv2 : zero));
     out[8] = lm * ((z ? dv1 : zero) + (y ? dv2 : zero));
@@ -224,8 +236,8 @@ __device__ __forceinline__ void lift_face(const CT *J, int ax, CT sg, CT L,
   {
     out[0] = Li * J[0];
     out[1] = Li * J[1];
-    out[2] = ll + (x ? two * lm * dv0 : zero);
-    out[3] = ll + (y ? two * lm * dv1 : zero);
+    out[2] = x ? fma_ct(two * lm, dv0, ll) : ll;
+    out[3] = y ? fma_ct(two * lm, dv1, ll) : ll;
     out[4] = lm * ((y ? dv0 : zero) + (x ? dv1 : zero));
   }
 }

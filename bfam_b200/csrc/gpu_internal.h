@@ -72,6 +72,7 @@ struct KernelSet
   int NT = 0;
   int occ[2] = {0, 0}; // resident CTAs per SM of the stage and rhs kernels
   int nbuf = 1;        // element buffers per CTA
+  int elements = 1;    // elements per CTA
 };
 
 // the kernels of one (dim, order, precision)

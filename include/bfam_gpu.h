@@ -430,7 +430,8 @@ int bfam_gpu_batch_add_pglue(bfam_gpu_batch_t *b, bfam_gpu_pglue_t *g);
  * register budget for `min_ctas` resident CTAs per SM.  Tile 0 is the
  * single-domain kernel's (one element per CTA).  At 3D orders 6 and 7 the
  * shapes are the precision form's; the plain form's tiles there are one warp
- * per plane of nodes. */
+ * per plane of nodes.  In 2D and at 3D orders 1 and 2 tile 0 packs several
+ * elements into a CTA, a thread per node, whatever shape it reports. */
 int bfam_gpu_tile_count(int dim, int N);
 int bfam_gpu_tile_shape(int dim, int N, int tile, int *threads,
                         int *min_ctas);
