@@ -176,7 +176,7 @@ template <int DIM, int N, typename CT> BatchTile first_tile()
                     CT>::make();
 }
 
-// the matrix-instruction kernel (plain form, 3D orders 6 and 7) with a register
+// the matrix-instruction kernel (plain form, 3D orders 5 to 7) with a register
 // budget for MINB resident CTAs per SM
 template <int N, int MINB> struct MmaTile
 {
@@ -282,18 +282,25 @@ template <typename CT> std::vector<BatchTile> tiles_for(int dim, int N)
   return v;
 }
 
-// the plain form's tiles at 3D orders 6 and 7, as many as the precision form
-// has: one kernel, at N = 7 also under a register budget for one CTA
+// the plain form's tiles under the matrix kernel, as many as the precision
+// form has: one kernel under several register budgets
 std::vector<BatchTile> mma_tiles(int N)
 {
+  if (N == 5)
+    return {MmaTile<5, MmaShape<5>::MINB>::make(), MmaTile<5, 4>::make(),
+            MmaTile<5, 3>::make(),                 MmaTile<5, 1>::make(),
+            MmaTile<5, 2>::make(),                 MmaTile<5, 2>::make()};
   if (N == 6)
     return {MmaTile<6, MmaShape<6>::MINB>::make()};
   return {MmaTile<7, MmaShape<7>::MINB>::make(), MmaTile<7, 1>::make()};
 }
 
-std::vector<BatchTile> tiles(int dim, int N, int precision)
+// hops: the group's operators (the node-per-thread kernel's table without)
+std::vector<BatchTile> tiles(int dim, int N, int precision,
+                             const double *hops = nullptr)
 {
-  if (dim == 3 && (N == 6 || N == 7) && precision != BFAM_GPU_PRECISION_FP32)
+  if (dim == 3 && precision != BFAM_GPU_PRECISION_FP32 &&
+      (N == 6 || N == 7 || (N == 5 && hops && mma_for_mesh<5>(hops))))
     return mma_tiles(N);
   return precision == BFAM_GPU_PRECISION_FP32 ? tiles_for<float>(dim, N)
                                               : tiles_for<double>(dim, N);
@@ -1041,11 +1048,12 @@ int bfam_gpu_batch_create(bfam_gpu_domain_t *const *doms, int ndom,
       G.precision = d->precision;
       G.flux = d->flux;
       G.hops = d->hops;
-      G.tiles = tiles(d->dim, d->N, d->precision);
-      // several domains at N = 5 in FP64: the four-CTA tile, whose batch
-      // kernel does not spill (104 against 100 G DOF-updates/s)
+      G.tiles = tiles(d->dim, d->N, d->precision, d->hops.data());
+      // several conforming domains at N = 5 in FP64: the four-CTA tile, whose
+      // batch kernel does not spill (104 against 100 G DOF-updates/s)
       G.multi_tile = d->dim == 3 && d->N == 5 &&
-                     d->precision == BFAM_GPU_PRECISION_FP64;
+                     d->precision == BFAM_GPU_PRECISION_FP64 &&
+                     !mma_for_mesh<5>(d->hops.data());
       if (G.tiles.empty())
       {
         batch_release(b);

@@ -60,21 +60,32 @@ constexpr auto single_kernel =
 template <int N, int MODE>
 constexpr auto mma_kernel = dg_mma_kernel<N, MmaShape<N>::MINB, MODE>;
 
+template <int N>
+cudaError_t mma_launch(const DomainView &v, int n, const StageParams &sp,
+                       const double *hops, int mode, cudaStream_t stream,
+                       bool overlap)
+{
+  using M = MmaShape<N>;
+  return launch_dependent(overlap,
+                          mode == MODE_RHS ? mma_kernel<N, MODE_RHS>
+                                           : mma_kernel<N, MODE_STAGE>,
+                          n, M::NT, M::BYTES, stream, v, n, sp,
+                          1.0 / hops[7 * (N + 1) * (N + 1)]);
+}
+
 // n work items on a persistent grid of `grid` CTAs
 template <int DIM, int N, typename CT>
 cudaError_t stage_launch(const DomainView &v, int n, const StageParams &sp,
                          const double *hops, int mode, int grid,
                          cudaStream_t stream, bool overlap)
 {
-  if constexpr (use_mma<DIM, N, CT>())
+  if constexpr (use_mma_hanging<DIM, N, CT>())
   {
-    using M = MmaShape<N>;
-    const double iwend = 1.0 / hops[7 * (N + 1) * (N + 1)];
-    return launch_dependent(overlap,
-                            mode == MODE_RHS ? mma_kernel<N, MODE_RHS>
-                                             : mma_kernel<N, MODE_STAGE>,
-                            grid, M::NT, M::BYTES, stream, v, n, sp, iwend);
+    if (mma_for_mesh<N>(hops))
+      return mma_launch<N>(v, n, sp, hops, mode, stream, overlap);
   }
+  if constexpr (use_mma<DIM, N, CT>())
+    return mma_launch<N>(v, n, sp, hops, mode, stream, overlap);
   else if constexpr (use_pack<DIM, N, CT>())
   {
     using K = PackShape<DIM, N, CT>;
@@ -146,6 +157,15 @@ template <int DIM, int N, typename CT> cudaError_t stage_prepare(int *occ)
     using S = Shape<DIM, N>;
     const size_t smem = stage_smem_bytes<DIM, N, CT>();
     cudaError_t e = allow_smem(single_kernel<DIM, N, CT, MODE_STAGE_NC>, (int)smem);
+    if constexpr (use_mma_hanging<DIM, N, CT>())
+    {
+      // as many resident CTAs in both kernels (MmaShape::MINB), so one
+      // lookahead serves them
+      if (e == cudaSuccess)
+        e = allow_smem(mma_kernel<N, MODE_STAGE>, (int)MmaShape<N>::BYTES);
+      if (e == cudaSuccess)
+        e = allow_smem(mma_kernel<N, MODE_RHS>, (int)MmaShape<N>::BYTES);
+    }
     if (e == cudaSuccess)
       e = occupancy(single_kernel<DIM, N, CT, MODE_STAGE>, S::NT, smem,
                     &occ[MODE_STAGE]);

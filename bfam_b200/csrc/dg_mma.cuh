@@ -1,4 +1,4 @@
-// Stage kernel of the plain (FP64) form for 3D orders 6 and 7: the fused
+// Stage kernel of the plain (FP64) form for 3D orders 5 to 7: the fused
 // element update of dg_stage.cuh with its small dense operators on the FP64
 // matrix instruction (mma.sync m8n8k4, the only tensor-core form of FP64).
 //
@@ -6,8 +6,9 @@
 // the lines of a plane or a face, so one warp holds one plane (or one face)
 // as an 8 x 8 matrix in the instruction's accumulator layout,
 //   lane 4 r + c holds X[r][2 c], X[r][2 c + 1]            ("C layout"),
-// rows the plane's second axis, columns its first; rows and columns past
-// N are zero.  The order of the contracted index is free as long as both
+// rows the plane's second axis, columns its first; past N lanes repeat the
+// last row or columns, which meet zeros in the operators' fragments or land
+// where nothing is stored.  The order of the contracted index is free as long as both
 // operands agree on it, so with kstep s taking the indices 2 c + s
 //   X D^T     takes the C layout of X as its left operand unchanged, and
 //   Op X^T    takes the C layout of X as its right operand unchanged;
@@ -38,14 +39,14 @@
 // x derivative reads each value once and its y and z derivatives twice
 // (8,100 warp instructions per N = 7 element instead of 19,300).  Measured
 // on 29-32 M DOF bricks, G DOF-updates/s before -> now, conforming and with
-// 30 % of the base cells refined: N = 7 131.9 -> 174.7 and 105.5 -> 147.4,
-// N = 6 75.0 -> 125.3 and 58.9 -> 109.7.  Orders below 6 keep the
+// 30 % of the base cells refined: N = 7 131.9 -> 180 and 105.5 -> 155, N = 6
+// 75.0 -> 130 and 58.9 -> 114; N = 5 with hanging faces 122 -> 127 (on 197 M
+// DOFs 116 -> 125).  Lower orders and conforming N = 5 keep the
 // node-per-thread kernel: their planes leave too much of an 8 x 8 matrix
-// empty (N = 5, 36 of 64 entries: 145 here against 160 conforming, 120
-// against 122 refined; N = 4: 98 against 95, 82 against 82).
-// What bounds it now is latency: two CTAs of 8 warps per SM (82 KB each), each
-// in turn waiting for its loads (5,000 cycles of 14,000), at 81 % and 69 % of
-// the HBM bandwidth.
+// empty (N = 4, 25 of 64 entries: 89 against 95 conforming).
+// What bounds it now is latency: two CTAs of 8 warps per SM at N = 7 (82 KB
+// each), each in turn waiting for its loads (4,700 cycles of 14,000), at 84 %
+// and 72 % of the HBM bandwidth.
 #pragma once
 
 #include "dg_common.cuh"
@@ -70,14 +71,33 @@ template <int N> struct MmaShape
   static constexpr int OFF_FC = OFF_J + 36 * P;
   static constexpr int OFF_BAR = OFF_FC + 32;
   static constexpr size_t BYTES = (OFF_BAR + 2) * sizeof(double);
-  static constexpr int MINB = N == 6 ? 3 : 2;
+  static constexpr int MINB = N == 5 ? 5 : N == 6 ? 3 : 2;
 };
 
-// orders and arithmetic the kernel serves
+// Orders and arithmetic the kernel serves: always at orders 6 and 7, and at
+// order 5 where the domain's mesh has hanging faces (mma_for_mesh): with 30 %
+// of the base cells refined 127 G DOF-updates/s here against 123.5 in the
+// node-per-thread kernel, conforming 155 against 162.
 template <int DIM, int N, typename CT>
 __host__ __device__ constexpr bool use_mma()
 {
   return DIM == 3 && N >= 6 && sizeof(CT) == sizeof(double);
+}
+template <int DIM, int N, typename CT>
+__host__ __device__ constexpr bool use_mma_hanging()
+{
+  return DIM == 3 && N == 5 && sizeof(CT) == sizeof(double);
+}
+// hops: the domain's operators Dr | interpolation[3] | projection[3] | w; a
+// domain without a glue grid has identities for interpolations
+template <int N> inline bool mma_for_mesh(const double *hops)
+{
+  constexpr int n = N + 1;
+  const double *bottom = hops + 2 * n * n;
+  for (int i = 0; i < n * n; ++i)
+    if (bottom[i] != (i % (n + 1) == 0 ? 1.0 : 0.0))
+      return true;
+  return false;
 }
 
 // d += a b, one 8 x 8 x 4 step
@@ -134,8 +154,8 @@ __device__ __forceinline__ void put2(double *p, const double2 x, bool v0, bool v
 }
 
 // L2 prefetch of what the CTA of a later work item will read of its element
-// e, a line of 128 bytes per thread: state and dq rows, face descriptors,
-// element data, flux constants and the mortar slots of its coarse faces.
+// e, a line of 128 bytes per thread: state and dq rows, element data and flux
+// constants.
 // (The bulk prefetches of prefetch_element, 21 from one thread at about 200
 // cycles each, held that thread's warp and with it the CTA's barriers: 4,300
 // of the 18,800 cycles of an N = 7 element's CTA.)
@@ -162,20 +182,10 @@ __device__ __forceinline__ void prefetch_lines(const DomainView &d,
         prefetch_l2(d.dq + at);
     }
   }
-  const int2 *desc = d.fdesc + (size_t)e * 6;
   if (t < 6)
     prefetch_l2(d.fcE + (size_t)e * 6 + t);
   else if (t == 6)
     prefetch_l2(d.ed + e);
-  constexpr int LM = (24 * P * 8 + 127) / 128;
-#pragma unroll 1
-  for (int f = 0; f < 6; ++f)
-  {
-    const int2 ds = desc[f];
-    if ((ds.y & 3) == 2)
-      for (int l = t; l < LM; l += NT)
-        prefetch_l2(d.mbuf + (size_t)ds.x * 6 * P + 16 * l);
-  }
 }
 
 // work item blockIdx.x of n
@@ -315,15 +325,21 @@ __device__ __forceinline__ void mma_element(const Item &item, int n,
     }
   }
   // a later item's element, while this one's loads fly
+  const int ia = blockIdx.x + sp.ahead;
+  int2 dsa = make_int2(0, 0); // its face w
+  if (sp.ahead > 0 && ia < n)
   {
-    const int ia = blockIdx.x + sp.ahead;
-    if (sp.ahead > 0 && ia < n)
-      prefetch_lines<N, MODE, M::NT>(item.view(ia), sp, item.elem(ia), t);
+    const int ea = item.elem(ia);
+    if (w < 6)
+      dsa = item.view(ia).fdesc[(size_t)ea * 6 + w];
+    prefetch_lines<N, MODE, M::NT>(item.view(ia), sp, ea, t);
+    if (t == 8 && ia + sp.ahead < n) // and the entry read here by that CTA
+      item.prefetch(ia + sp.ahead);
   }
   // fragments of D, zero past N: for X D^T and Op X^T (column 2 c + s), and
   // along y and z, whose right operands are read from shared memory, with
   // the contracted index that meets fewer bank conflicts (2 c + s or c + 4 s)
-  constexpr bool YS = N == 7, ZS = N == 7;
+  constexpr bool YS = N == 7, ZS = N == 7 || N == 5;
   auto dfrag = [&](int k) {
     return rr < Nq && k < Nq ? __ldg(d.ops + rr + Nq * k) : 0.0;
   };
@@ -477,6 +493,15 @@ __device__ __forceinline__ void mma_element(const Item &item, int n,
         put2<VEC>(o + q * P, nb[q], v0, v1);
     }
   }
+  // the later item's mortar slots of a coarse face (its descriptor, a trip to
+  // memory, has arrived by now: read ahead of the prefetches face by face,
+  // six such trips in a row held the CTA)
+  if ((dsa.y & 3) == 2)
+  {
+    constexpr int L = (24 * P * 8 + 127) / 128;
+    for (int l = t & 31; l < L; l += 32)
+      prefetch_l2(item.view(ia).mbuf + (size_t)dsa.x * 6 * P + 16 * l);
+  }
   const double2 fx = make_double2(dfrag(2 * c), dfrag(2 * c + 1));
   const double2 fy = YS ? make_double2(dfrag(c), dfrag(c + 4)) : fx;
   __syncthreads();
@@ -510,7 +535,9 @@ __device__ __forceinline__ void mma_element(const Item &item, int n,
     return y;
   };
   auto dxy = [&](int f, int jx, int g, int jy, double2 &X, double2 &Y) {
-    const double2 x = get2<VEC>(row(f) + m0, o1);
+    double2 x = make_double2(0.0, 0.0);
+    if (rr < Nq)
+      x = get2<VEC>(row(f) + m0, o1);
     X = startx(jx);
     Y = starty(jy);
     dmma(X, x.x, fx.x);
@@ -522,7 +549,9 @@ __device__ __forceinline__ void mma_element(const Item &item, int n,
   const double *pz = zrow(0, w, r) + i0;
   const double *jz = pt + (w == N ? 30 : 24) * P + i0 + Nq * r;
   auto dz = [&](int q, int jq) {
-    double2 y = get2<VEC>(pz + q * Np, o1);
+    double2 y = make_double2(0.0, 0.0);
+    if (rr < Nq)
+      y = get2<VEC>(pz + q * Np, o1);
     if (w == 0 || w == N)
     {
       const double2 j = get2<VEC>(jz + jq * P, o1);
@@ -536,8 +565,11 @@ __device__ __forceinline__ void mma_element(const Item &item, int n,
   auto load_dq = [&](int f0, double2 *u) {
 #pragma unroll
     for (int k = 0; k < 3; ++k)
-      u[k] = MODE != MODE_RHS && rd ? get2<VEC>(dqp + (f0 + k) * fs, o1)
-                                    : make_double2(0.0, 0.0);
+    {
+      u[k] = make_double2(0.0, 0.0);
+      if (MODE != MODE_RHS && rd && rr < Nq)
+        u[k] = get2<VEC>(dqp + (f0 + k) * fs, o1);
+    }
   };
   auto put = [&](int f0, const double2 *u) {
     const size_t at = eoff + n0 + f0 * fs;
@@ -549,16 +581,16 @@ __device__ __forceinline__ void mma_element(const Item &item, int n,
     }
     else
     {
-      double2 o[3];
-#pragma unroll
-      for (int k = 0; k < 3; ++k)
-      {
-        const double2 q = get2<VEC>(row(f0 + k) + m0, o1);
-        o[k] = make_double2(q.x + sp.B * u[k].x, q.y + sp.B * u[k].y);
-      }
       // streaming stores, as in dg_stage.cuh
       if (v0)
       {
+        double2 o[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+        {
+          const double2 q = get2<VEC>(row(f0 + k) + m0, o1);
+          o[k] = make_double2(q.x + sp.B * u[k].x, q.y + sp.B * u[k].y);
+        }
 #pragma unroll
         for (int k = 0; k < 3; ++k)
         {

@@ -3,8 +3,8 @@
 //
 // One element per CTA iteration does:
 //   issue   : every global read of the element is issued up front -- its own
-//             q (and dq, where the shape stages it; else an L2 prefetch of
-//             it) and its faces' flux constants by TMA bulk copies into
+//             q (and dq, where the shape stages it) and its faces' flux
+//             constants by TMA bulk copies into
 //             shared memory, the neighbours' face traces by 8-byte cp.async
 //             gathers straight into shared memory, addressed from a
 //             per-face descriptor.  This is the
@@ -103,7 +103,9 @@ template <int DIM, int N, typename CT, int NBUF, bool DQS = true> struct Tile
 {
   using S = Shape<DIM, N>;
   // DQS: the element's dq rows are staged in shared memory (TMA); otherwise
-  // they are prefetched into L2 and read from global memory by the update
+  // they are read from global memory by the update, in L2 by the lookahead of
+  // an earlier CTA (prefetching them once more with the element's own loads
+  // cost 1-2 % at N = 5 and 7)
   static constexpr int BUF =
       S::SM_QS + (DQS ? S::SM_DQ : 0) + S::SM_PT + 4 * S::NF;
   static constexpr int OFF_MJ = NBUF * BUF;
@@ -135,8 +137,7 @@ __host__ __device__ constexpr int resident_ctas()
 
 // dq staged in shared memory (TMA) unless the shape reads it from L2 in the
 // update (Shape::DQ_L2 / DQ_L2_NARROW: 3D N=7, and the precision form at
-// 3D N=5, where staging measured 9 % slower; the rows are prefetched into
-// L2 when the element's loads are issued), or unless leaving it out admits
+// 3D N=5, where staging measured 9 % slower), or unless leaving it out admits
 // more resident CTAs (the plain form at 3D N=5: five CTAs instead of four)
 template <int DIM, int N, typename CT> __host__ __device__ constexpr bool stage_dqs()
 {
@@ -265,12 +266,6 @@ __device__ __forceinline__ void issue_element(const DomainView &d,
           for (int c = 0; c < NFLD; ++c)
             bulk_g2s(R + c * Np, d.dq + c * fs + eoff, Np * sizeof(double),
                      bar_dq);
-        }
-        else
-        {
-#pragma unroll
-          for (int c = 0; c < NFLD; ++c)
-            bulk_prefetch_l2(d.dq + c * fs + eoff, Np * sizeof(double));
         }
       }
     }
@@ -749,6 +744,12 @@ struct SingleItems
   {
     return d.elist ? d.elist[idx] : idx;
   }
+  // the item's own entry into L2
+  __device__ __forceinline__ void prefetch(int idx) const
+  {
+    if (d.elist)
+      prefetch_l2(d.elist + idx);
+  }
 };
 
 // many domains: item idx is work[idx] = (domain, element)
@@ -761,6 +762,10 @@ struct BatchItems
     return views[work[idx].x];
   }
   __device__ __forceinline__ int elem(int idx) const { return work[idx].y; }
+  __device__ __forceinline__ void prefetch(int idx) const
+  {
+    prefetch_l2(work + idx);
+  }
 };
 
 // One domain: item idx is element idx, or the idx-th of the launch's

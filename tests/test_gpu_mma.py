@@ -1,4 +1,5 @@
-"""The matrix-instruction stage kernel (plain form, 3D orders 6 and 7) at the
+"""The matrix-instruction stage kernel (plain form, 3D orders 6 and 7, and
+order 5 on meshes with hanging faces) at the
 sizes where its copies and its layout can go wrong, against the oracle: a
 single element that is its own neighbour, odd and even element counts (rows
 of an odd number of nodes start off the 16-byte boundary in alternation, and
@@ -29,7 +30,7 @@ CASES = [
 ]
 
 
-@pytest.mark.parametrize("N", [6, 7])
+@pytest.mark.parametrize("N", [5, 6, 7])
 @pytest.mark.parametrize("case", CASES, ids=lambda c: f"{c[0]}-p{c[1]}-b{int(c[3])}")
 @pytest.mark.parametrize("flux", [bf.FLUX_UPWIND, bf.FLUX_CENTRAL], ids=["upwind", "central"])
 def test_mma_kernel_against_the_oracle(N, case, flux):
@@ -54,7 +55,7 @@ def test_mma_kernel_against_the_oracle(N, case, flux):
     b.free()
 
 
-@pytest.mark.parametrize("N", [6, 7])
+@pytest.mark.parametrize("N", [5, 6, 7])
 def test_mma_kernel_point_source(N):
     m = bf.Mesh(3, N, (2, 2, 1), refine_prob=0.5, seed=4)
     rho, lam, mu = bf.material_random(m.K, 4)
