@@ -152,14 +152,24 @@ template <int DIM, int N> struct Shape
   //     (109.1-109.4 vs 105.1-105.3 with seven; 105.6 with twelve), twelve
   //     in the precision form, which then reads dq from L2 (115.4 vs 104.3
   //     with seven, 109.2 with ten);
-  //   3D N=7: two CTAs of 384 threads (three: 92.2 vs 102.3, spills).
+  //   3D N=4: six CTAs of 160 threads in the plain form (137 conforming and
+  //     106 refined; four 128 and 94, seven 132 and 100, eight 134 and 104),
+  //     seven in the precision form (156 and 117; four 134 and 96, six 143
+  //     and 104, eight 134 and 101);
+  //   3D N=6, precision form: three CTAs of 352 threads with one buffer (141
+  //     and 112; two CTAs 129 and 98, one with two buffers 106 and 74);
+  //   3D N=7, precision form: two CTAs of 384 threads (three: 92.2 vs 102.3,
+  //     spills).
   static constexpr int MINB_RAW = 65536 / (NT * 96);
   static constexpr int MINB =
       (DIM == 3 && N == 7)   ? 2
       : (DIM == 3 && N == 5) ? 5
+      : (DIM == 3 && N == 4) ? 6
       : (DIM == 3 && N == 3) ? 10
                              : (MINB_RAW < 1 ? 1 : (MINB_RAW > 16 ? 16 : MINB_RAW));
   static constexpr int MINB_NARROW = (DIM == 3 && N == 5)   ? 4
+                                     : (DIM == 3 && N == 4) ? 7
+                                     : (DIM == 3 && N == 6) ? 3
                                      : (DIM == 3 && N == 3) ? 12
                                                             : MINB;
   // dq read from global memory (L2) in the update instead of staged in
@@ -168,9 +178,16 @@ template <int DIM, int N> struct Shape
   // DOF-updates/s in the plain form), and in the precision form at N=5
   static constexpr bool DQ_L2 = DIM == 3 && N == 7;
   static constexpr bool DQ_L2_NARROW = DIM == 3 && N == 5;
-  static constexpr bool TMA = (Np % 2) == 0; // 16-byte aligned element rows
+  // Element rows of an odd number of nodes start on an 8-byte boundary in
+  // global memory for every other element (and, with an odd number of
+  // elements, every other field); the bulk copy of such a row starts at the
+  // 16-byte boundary below and takes one value more, so a field's row in
+  // shared memory is PITCH long and starts at RowShift's 0 or 1.  (With
+  // 8-byte cp.async copies of these rows, four CTAs at N = 4 did 95 G
+  // DOF-updates/s conforming and 82 refined, against 128 and 94.)
+  static constexpr int PITCH = Np + Np % 2;
   // shared memory regions in doubles (all even, so 16-byte aligned)
-  static constexpr int SM_QS = NFLD * Np + (NFLD * Np) % 2; // q
+  static constexpr int SM_QS = NFLD * PITCH; // q
   static constexpr int SM_DQ = SM_QS; // dq, then A dq + dt rhs in place
   // per face: the neighbour's NTF trace fields, then in place the NJ flux
   // jumps of each face node (NJ == NTF)
@@ -185,6 +202,20 @@ template <int DIM, int N> struct Shape
   // precision form only: FP32 copy of q minus the element's first node,
   // after the mbarriers
   static constexpr int SM_QF = (NFLD * Np + 3) / 4 * 2;
+};
+
+// where an element's field rows start in their PITCH-long slots
+template <int Np> struct RowShift
+{
+  int even, odd; // fields of even and odd number
+  __device__ __forceinline__ RowShift(int32_t K, int e)
+      : even(Np % 2 ? e & 1 : 0), odd(Np % 2 ? (e + K) & 1 : 0)
+  {
+  }
+  __device__ __forceinline__ int operator()(int c) const
+  {
+    return c & 1 ? odd : even;
+  }
 };
 
 // ------------------------------------------------------------ PTX helpers

@@ -390,7 +390,8 @@ __device__ __forceinline__ void pack_elements(const Item &item, int n,
   const ElemData &me = ed[ms];
   const int i = mn % Nq, j = (mn / Nq) % Nq, k = mn / (Nq * Nq);
   CT rv[NFLD];
-  volume_node<DIM, N, CT, NV>(qv + ms * Np, sD, dop, me, s, i, j, k, rv);
+  volume_node<DIM, N, CT>([&](int c) { return qv + c * NV + ms * Np; }, sD, dop,
+                          me, s, i, j, k, rv);
 #pragma unroll
   for (int ax = 0; ax < DIM; ++ax)
   {

@@ -235,7 +235,7 @@ __device__ __forceinline__ void issue_element(const DomainView &d,
 {
   using S = Shape<DIM, N>;
   constexpr int Np = S::Np, Nfp = S::Nfp, NF = S::NF, NFLD = S::NFLD,
-                NTF = S::NTF;
+                NTF = S::NTF, PITCH = S::PITCH;
   const TileBuf<DIM, N, CT, NBUF, NT, EPC> tb(b);
   double *qs = tb.qs, *R = tb.R, *pt = tb.pt, *fcf = tb.fcf;
   uint64_t *bar_q = tb.bq, *bar_dq = tb.bdq;
@@ -244,39 +244,30 @@ __device__ __forceinline__ void issue_element(const DomainView &d,
   const size_t eoff = (size_t)e * Np;
   const bool rd = MODE != MODE_RHS && !sp.first_stage;
   const int2 *desc = d.fdesc + (size_t)e * NF;
-  if constexpr (S::TMA)
+  if (t == 0)
   {
-    if (t == 0)
-    {
-      fence_proxy_async(); // shared memory of the previous element is free
-      mbar_expect_tx(bar_q, NFLD * Np * sizeof(double) + NF * sizeof(double4));
+    const RowShift<Np> sh(d.K, e);
+    // row c of `src` to its slot; the last row of an odd-sized array has no
+    // value after it to copy, and its own last one goes by itself
+    const bool last = Np % 2 && e == d.K - 1 && (d.K & 1);
+    auto rows = [&](double *dst, const double *src, uint64_t *bar, int more) {
+      if (last)
+        dst[(NFLD - 1) * PITCH + Np - 1] = src[(NFLD - 1) * fs + eoff + Np - 1];
+      mbar_expect_tx(bar, (NFLD * PITCH - (last ? 2 : 0) + more) * sizeof(double));
 #pragma unroll
       for (int c = 0; c < NFLD; ++c)
-        bulk_g2s(qs + c * Np, d.qin + c * fs + eoff, Np * sizeof(double),
-                 bar_q);
-      // the face flux constants with the state, so that no thread needs
-      // another thread's copies before the face phase
-      bulk_g2s(fcf, d.fcE + (size_t)e * NF, NF * sizeof(double4), bar_q);
-      if (rd)
-      {
-        if constexpr (stage_dqs<DIM, N, CT>())
-        {
-          mbar_expect_tx(bar_dq, NFLD * Np * sizeof(double));
-#pragma unroll
-          for (int c = 0; c < NFLD; ++c)
-            bulk_g2s(R + c * Np, d.dq + c * fs + eoff, Np * sizeof(double),
-                     bar_dq);
-        }
-      }
-    }
-  }
-  else
-  {
-    for (int w = t; w < NFLD * Np; w += NT)
+        bulk_g2s(dst + c * PITCH, src + c * fs + eoff - sh(c),
+                 (PITCH - (last && c == NFLD - 1 ? 2 : 0)) * sizeof(double), bar);
+    };
+    fence_proxy_async(); // shared memory of the previous element is free
+    // the face flux constants with the state, so that no thread needs
+    // another thread's copies before the face phase
+    rows(qs, d.qin, bar_q, 4 * NF);
+    bulk_g2s(fcf, d.fcE + (size_t)e * NF, NF * sizeof(double4), bar_q);
+    if constexpr (stage_dqs<DIM, N, CT>())
     {
-      cp_async8(qs + w, d.qin + (w / Np) * fs + eoff + (w % Np));
-      if (stage_dqs<DIM, N, CT>() && rd)
-        cp_async8(R + w, d.dq + (w / Np) * fs + eoff + (w % Np));
+      if (rd)
+        rows(R, d.dq, bar_dq, 0);
     }
   }
 
@@ -303,15 +294,8 @@ __device__ __forceinline__ void issue_element(const DomainView &d,
                   src + trace_field<DIM>(f >> 1, c) * fs);
       }
     }
-    if (!S::TMA && pn == 0)
-    {
-      const double *fc =
-          reinterpret_cast<const double *>(d.fcE + (size_t)e * NF + f);
-      cp_async16(fcf + 4 * f, fc);
-      cp_async16(fcf + 4 * f + 2, fc + 2);
-    }
   }
-  cp_async_commit(); // own state and constants (non-TMA path), face traces
+  cp_async_commit(); // the face traces
 
 }
 
@@ -323,19 +307,20 @@ __device__ __forceinline__ void prefetch_element(const DomainView &d,
                                                  const StageParams &sp, int e)
 {
   using S = Shape<DIM, N>;
-  if constexpr (S::TMA)
   {
     constexpr int Np = S::Np, NF = S::NF, NFLD = S::NFLD;
     const size_t eoff = (size_t)e * Np;
-#pragma unroll
-    for (int c = 0; c < NFLD; ++c)
-      bulk_prefetch_l2(d.qin + c * d.fs + eoff, Np * sizeof(double));
-    if (MODE != MODE_RHS && !sp.first_stage)
-    {
+    const RowShift<Np> sh(d.K, e);
+    // the 16-byte aligned part of each row, never past its end
+    auto rows = [&](const double *src) {
 #pragma unroll
       for (int c = 0; c < NFLD; ++c)
-        bulk_prefetch_l2(d.dq + c * d.fs + eoff, Np * sizeof(double));
-    }
+        bulk_prefetch_l2(src + c * d.fs + eoff - sh(c),
+                         (Np % 2 ? Np - 1 + 2 * sh(c) : Np) * sizeof(double));
+    };
+    rows(d.qin);
+    if (MODE != MODE_RHS && !sp.first_stage)
+      rows(d.dq);
     bulk_prefetch_l2(d.fdesc + (size_t)e * NF, NF * sizeof(int2));
     bulk_prefetch_l2(d.ed + e, sizeof(ElemData));
     bulk_prefetch_l2(d.fcE + (size_t)e * NF, NF * sizeof(double4));
@@ -368,14 +353,18 @@ __device__ __forceinline__ void compute_element(const DomainView &d,
   using T = Tile<DIM, N, CT, NBUF, stage_dqs<DIM, N, CT>()>;
   constexpr int Nq = S::Nq, Np = S::Np, Nfp = S::Nfp, NF = S::NF,
                 NFLD = S::NFLD, NJ = S::NJ, NPC = S::NPC, ROWS = S::ROWS,
-                NTF = S::NTF;
+                NTF = S::NTF, PITCH = S::PITCH;
   // this sub-element's tile, derived from the dynamic shared array itself
   // (not a pointer parameter), so that all accesses stay in the shared
   // window with 32-bit addressing
   double *smem = sub_smem<T, NT, EPC>();
   const TileBuf<DIM, N, CT, NBUF, NT, EPC> tb(b);
-  double *qs = tb.qs, *R = tb.R, *pt = tb.pt, *fcf = tb.fcf;
+  double *qs = tb.qs, *pt = tb.pt, *fcf = tb.fcf;
   uint64_t *bar_q = tb.bq, *bar_dq = tb.bdq;
+  // field rows of the state and of dq
+  const RowShift<Np> sh(d.K, e);
+  auto row = [&](int c) { return qs + c * PITCH + sh(c); };
+  auto dq_row = [&](int c) { return tb.R + c * PITCH + sh(c); };
   double *mj = smem + T::OFF_MJ; // [DIM][NJ][Nfp] coarse-side jumps, by fine rank
   const CT *sD = reinterpret_cast<const CT *>(smem + T::OFF_OPS); // D
   // the volume pass's copy of q: q itself in the plain form; in the
@@ -383,11 +372,9 @@ __device__ __forceinline__ void compute_element(const DomainView &d,
   // derivative of a constant is zero), so that rounding is relative to the
   // variation inside the element
   constexpr bool NARROW = T::NARROW;
-  CT *qv;
+  CT *qv = nullptr;
   if constexpr (NARROW)
     qv = reinterpret_cast<CT *>(smem + T::OFF_QV);
-  else
-    qv = qs;
 
   const int t = Sub<NT, EPC>::t();
   const size_t fs = d.fs;
@@ -410,27 +397,22 @@ __device__ __forceinline__ void compute_element(const DomainView &d,
   const int ncoarse = __popc(coarse_mask), nfine = __popc(fine_mask);
 
   // ------------------------------------------------- phase 1: faces, mortars
-  if constexpr (S::TMA)
-  {
-    if (!mbar_wait(bar_q, par))
-      atomicExch(d.err, 1);
-  }
+  if (!mbar_wait(bar_q, par))
+    atomicExch(d.err, 1);
   cp_async_wait<NBUF - 1>(); // this element's group (the next one may fly)
-  if constexpr (NARROW && !S::TMA)
-    Sub<NT, EPC>::sync(); // other threads' cp.async writes of q
   if constexpr (NARROW)
   {
     for (int n = t; n < Np; n += NT)
     {
 #pragma unroll
       for (int c = 0; c < NFLD; ++c)
-        qv[c * Np + n] = CT(qs[c * Np + n] - qs[c * Np]);
+        qv[c * Np + n] = CT(row(c)[n] - row(c)[0]);
     }
   }
-  // With the state and flux constants by TMA, a thread's face pass reads
+  // The state and flux constants come by TMA, and a thread's face pass reads
   // only its own gathered trace slots (its own cp.async group), so only the
   // fine-side interpolation, which reads whole lines, needs the barrier.
-  if (!S::TMA || nfine)
+  if (nfine)
     Sub<NT, EPC>::sync();
   // lift factor of face axis ax: s (2/h_ax) / w_0
   CT lfac[3];
@@ -487,7 +469,7 @@ __device__ __forceinline__ void compute_element(const DomainView &d,
 #pragma unroll
         for (int c = 0; c < NTF; ++c)
         {
-          const double qm = qs[trace_field<DIM>(f >> 1, c) * Np + vm];
+          const double qm = row(trace_field<DIM>(f >> 1, c))[vm];
           const int g = f * NTF + c;
           const double qp = k != 3 ? pt[g * Nfp + fpos<DIM, N>(g, pp)]
                                    : (free_surface ? (c < DIM ? qm : -qm) : 0.0);
@@ -582,11 +564,8 @@ __device__ __forceinline__ void compute_element(const DomainView &d,
   constexpr bool DQS = stage_dqs<DIM, N, CT>();
   if (MODE != MODE_RHS && rd && DQS)
   {
-    if constexpr (S::TMA)
-    {
-      if (!mbar_wait(bar_dq, par))
-        atomicExch(d.err, 2);
-    }
+    if (!mbar_wait(bar_dq, par))
+      atomicExch(d.err, 2);
   }
   constexpr int NODE_ITERS = (Np + NT - 1) / NT;
 #pragma unroll 1
@@ -600,7 +579,11 @@ __device__ __forceinline__ void compute_element(const DomainView &d,
     // jumps of the faces this node lies on (at most one per axis, in face
     // order); widened to FP64 once for the update
     CT rv[NFLD];
-    volume_node<DIM, N, CT>(qv, sD, dop, me, s, i, j, k, rv);
+    if constexpr (NARROW)
+      volume_node<DIM, N, CT>([&](int c) { return qv + c * Np; }, sD, dop, me, s,
+                              i, j, k, rv);
+    else
+      volume_node<DIM, N, CT>(row, sD, dop, me, s, i, j, k, rv);
 #pragma unroll
     for (int ax = 0; ax < DIM; ++ax)
     {
@@ -643,7 +626,7 @@ __device__ __forceinline__ void compute_element(const DomainView &d,
       {
 #pragma unroll
         for (int c = 0; c < NFLD; ++c)
-          acc[c] += a * (DQS ? R[c * Np + n] : d.dq[c * fs + eoff + n]);
+          acc[c] += a * (DQS ? dq_row(c)[n] : d.dq[c * fs + eoff + n]);
       }
       // streaming stores: the next stage reads these rows a whole stage
       // later (from DRAM), so they should not push the lines in reuse out
@@ -652,7 +635,7 @@ __device__ __forceinline__ void compute_element(const DomainView &d,
       for (int c = 0; c < NFLD; ++c)
       {
         __stcs(d.dq + c * fs + eoff + n, acc[c]);
-        __stcs(d.qout + c * fs + eoff + n, qs[c * Np + n] + sp.B * acc[c]);
+        __stcs(d.qout + c * fs + eoff + n, row(c)[n] + sp.B * acc[c]);
       }
     }
     else

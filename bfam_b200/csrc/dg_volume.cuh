@@ -89,12 +89,11 @@ template <int DIM, int N, typename CT> constexpr int dparam_axes()
 //   rho dv/dt = div S,  dS/dt = lambda div(v) I + mu (grad v + grad v^T)
 // with the derivative along each axis the 1-D LGL differentiation matrix
 // applied along that axis -- the BFAM_KRON_IXIXA / IXAXI / AXIXI
-// contractions of src/bfam.c:3519-3624 evaluated at one node.  qs is the
-// element's state tile in CT, sD the column-major D(i,m) = sD[i + Nq m], both
+// contractions of src/bfam.c:3519-3624 evaluated at one node.  row(c) is the
+// element's field c in CT, sD the column-major D(i,m) = sD[i + Nq m], both
 // in shared memory, dop the same operators in the kernel's parameter space.
-// FS separates the fields in the tile.
-template <int DIM, int N, typename CT, int FS = Shape<DIM, N>::Np>
-__device__ __forceinline__ void volume_node(const CT *qs, const CT *sD,
+template <int DIM, int N, typename CT, typename Rows>
+__device__ __forceinline__ void volume_node(const Rows &row, const CT *sD,
                                             const DiffOp<N, CT> &dop,
                                             const ElemData &me, double s, int i,
                                             int j, int k, CT *rv)
@@ -110,10 +109,10 @@ __device__ __forceinline__ void volume_node(const CT *qs, const CT *sD,
   // derivative of field c along axis ax at this node
   auto deriv = [&](int c, int ax, const CT *Dl) {
     if (ax == 0)
-      return line_dx<N, CT>(qs + c * FS + Nq * (j + Nq * k), Dl);
+      return line_dx<N, CT>(row(c) + Nq * (j + Nq * k), Dl);
     if (ax == 1)
-      return line_ds<N, Nq, CT>(qs + c * FS + i + Nq * Nq * k, Dl);
-    return line_ds<N, Nq * Nq, CT>(qs + c * FS + i + Nq * j, Dl);
+      return line_ds<N, Nq, CT>(row(c) + i + Nq * Nq * k, Dl);
+    return line_ds<N, Nq * Nq, CT>(row(c) + i + Nq * j, Dl);
   };
 
   constexpr int PA = dparam_axes<DIM, N, CT>();
