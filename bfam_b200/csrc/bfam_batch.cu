@@ -48,6 +48,14 @@ struct BatchTile
   // whose elements have no coarse-side hanging face (level 0 of domains
   // without faces glued to another order)
   batch_launch_fn launch_nc = nullptr;
+  // and without any mortar pass, for domains without hanging faces
+  batch_launch_fn launch_cf = nullptr;
+  batch_launch_fn of(int mode) const
+  {
+    return mode == MODE_STAGE_CF ? launch_cf
+           : mode == MODE_STAGE_NC ? launch_nc
+                                   : launch;
+  }
   batch_prepare_fn prepare = nullptr;
   batch_occupancy_fn occupancy = nullptr;
 };
@@ -56,43 +64,37 @@ template <int DIM, int N, int NT, int MINB, typename CT, int EPC = 1>
 struct TileImpl
 {
   static constexpr int NB = EPC == 1 ? nbuf<DIM, N, CT>() : 1;
+  template <int MODE>
   static constexpr auto kernel =
-      dg_stage_batch_kernel<DIM, N, NT, MINB, MODE_STAGE, CT, NB, EPC>;
-  static constexpr auto kernel_nc =
-      dg_stage_batch_kernel<DIM, N, NT, MINB, MODE_STAGE_NC, CT, NB, EPC>;
+      dg_stage_batch_kernel<DIM, N, NT, MINB, MODE, CT, NB, EPC>;
   static constexpr size_t SMEM = stage_smem_bytes<DIM, N, CT, EPC>();
-  static cudaError_t launch(const DomainView *v, const int2 *w, int nwork,
-                     const StageParams &sp, const double *hops, int grid,
-                     cudaStream_t st, bool overlap)
+  template <int MODE>
+  static cudaError_t run(const DomainView *v, const int2 *w, int nwork,
+                         const StageParams &sp, const double *hops, int grid,
+                         cudaStream_t st, bool overlap)
   {
     const DiffOp<N, CT> dop = make_diffop<N, CT>(hops);
-    return launch_dependent(overlap, kernel, grid, NT * EPC, SMEM, st, v, w, nwork, sp,
-                            dop);
+    return launch_dependent(overlap, kernel<MODE>, grid, NT * EPC, SMEM, st, v,
+                            w, nwork, sp, dop);
   }
-  static cudaError_t launch_nc(const DomainView *v, const int2 *w, int nwork,
-                        const StageParams &sp, const double *hops, int grid,
-                        cudaStream_t st, bool overlap)
+  template <int MODE> static cudaError_t allow()
   {
-    const DiffOp<N, CT> dop = make_diffop<N, CT>(hops);
-    return launch_dependent(overlap, kernel_nc, grid, NT * EPC, SMEM, st, v, w, nwork,
-                            sp, dop);
+    return cudaFuncSetAttribute((const void *)kernel<MODE>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)SMEM);
   }
   static cudaError_t prepare()
   {
-    cudaError_t e = cudaFuncSetAttribute(
-        (const void *)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-        (int)SMEM);
-    if (e != cudaSuccess)
-      return e;
-    return cudaFuncSetAttribute((const void *)kernel_nc,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)SMEM);
+    cudaError_t e = allow<MODE_STAGE>();
+    if (e == cudaSuccess)
+      e = allow<MODE_STAGE_NC>();
+    return e == cudaSuccess ? allow<conforming_mode<DIM, N, CT>()>() : e;
   }
   static int occupancy()
   {
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, NT * EPC,
-                                                      SMEM) != cudaSuccess)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+            &n, kernel<MODE_STAGE>, NT * EPC, SMEM) != cudaSuccess)
     {
       cudaGetLastError();
       return 0;
@@ -106,8 +108,9 @@ struct TileImpl
     t.MINB = MINB;
     t.EPC = EPC;
     t.NBUF = NB;
-    t.launch = launch;
-    t.launch_nc = launch_nc;
+    t.launch = run<MODE_STAGE>;
+    t.launch_nc = run<MODE_STAGE_NC>;
+    t.launch_cf = run<conforming_mode<DIM, N, CT>()>;
     t.prepare = prepare;
     t.occupancy = occupancy;
     return t;
@@ -119,6 +122,12 @@ struct TileImpl
 template <int DIM, int N, typename CT> struct PackTile
 {
   using K = PackShape<DIM, N, CT>;
+  template <int MODE> static cudaError_t allow()
+  {
+    return cudaFuncSetAttribute(
+        (const void *)dg_pack_batch_kernel<DIM, N, MODE, CT>,
+        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)K::BYTES);
+  }
   template <int MODE>
   static cudaError_t run(const DomainView *v, const int2 *w, int nwork,
                          const StageParams &sp, const double *hops, int,
@@ -131,14 +140,10 @@ template <int DIM, int N, typename CT> struct PackTile
   }
   static cudaError_t prepare()
   {
-    cudaError_t e = cudaFuncSetAttribute(
-        (const void *)dg_pack_batch_kernel<DIM, N, MODE_STAGE, CT>,
-        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)K::BYTES);
-    return e != cudaSuccess
-               ? e
-               : cudaFuncSetAttribute(
-                     (const void *)dg_pack_batch_kernel<DIM, N, MODE_STAGE_NC, CT>,
-                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)K::BYTES);
+    cudaError_t e = allow<MODE_STAGE>();
+    if (e == cudaSuccess)
+      e = allow<MODE_STAGE_NC>();
+    return e == cudaSuccess ? allow<MODE_STAGE_CF>() : e;
   }
   static int occupancy()
   {
@@ -160,6 +165,7 @@ template <int DIM, int N, typename CT> struct PackTile
     t.pack = K::E;
     t.launch = run<MODE_STAGE>;
     t.launch_nc = run<MODE_STAGE_NC>;
+    t.launch_cf = run<MODE_STAGE_CF>;
     t.prepare = prepare;
     t.occupancy = occupancy;
     return t;
@@ -211,7 +217,7 @@ template <int N, int MINB> struct MmaTile
     BatchTile t;
     t.NT = M::NT;
     t.MINB = MINB;
-    t.launch = t.launch_nc = launch;
+    t.launch = t.launch_nc = t.launch_cf = launch;
     t.prepare = prepare;
     t.occupancy = occupancy;
     return t;
@@ -447,6 +453,7 @@ struct bfam_gpu_batch
     // no domain of the group has faces glued to another order, so level 0
     // holds no element with a coarse-side face (launched without that pass)
     bool level0_nc = false;
+    bool conforming = false; // nor any domain hanging faces
     cudaStream_t stream = nullptr;
     cudaEvent_t done = nullptr;
   };
@@ -626,7 +633,9 @@ cudaError_t launch_post_step(bfam_gpu_batch_t *b, int p)
 int launch_level(bfam_gpu_batch_t *b, bfam_gpu_batch::Group &g, size_t l,
                  int par, const StageParams &sp, cudaStream_t st, bool overlap)
 {
-  const bool nc = l == 0 && g.level0_nc;
+  const int mode = l > 0 || !g.level0_nc ? MODE_STAGE
+                   : g.conforming         ? MODE_STAGE_CF
+                                          : MODE_STAGE_NC;
   if (g.doms.size() == 1 && g.tile == 0 && g.ctas_per_sm == 0)
   {
     const int i = g.doms[0];
@@ -636,14 +645,12 @@ int launch_level(bfam_gpu_batch_t *b, bfam_gpu_batch::Group &g, size_t l,
     if (d->nlevels > 1)
       v.elist = d->elist + d->level_off[l];
     CUDA_TRY(d->ks.launch(v, (int)g.nwork_l[l], sp, g.hops.data(),
-                          nc ? MODE_STAGE_NC : MODE_STAGE, g.grid[l], st,
-                          overlap));
+                          mode, g.grid[l], st, overlap));
     return 0;
   }
   const BatchTile &t = g.tiles[g.tile];
-  CUDA_TRY((nc ? t.launch_nc : t.launch)(g.views[par], g.work[l],
-                                         (int)g.nwork_l[l], sp, g.hops.data(),
-                                         g.grid[l], st, overlap));
+  CUDA_TRY(t.of(mode)(g.views[par], g.work[l], (int)g.nwork_l[l], sp,
+                      g.hops.data(), g.grid[l], st, overlap));
   return 0;
 }
 
@@ -1084,6 +1091,7 @@ int bfam_gpu_batch_create(bfam_gpu_domain_t *const *doms, int ndom,
       if (doms[i]->nglued)
         G.level0_nc = false;
     }
+    G.conforming = nl == 1;
     for (int l = 0; l < nl; ++l)
     {
       // level l of every domain, domain-major

@@ -94,6 +94,7 @@ cudaError_t stage_launch(const DomainView &v, int n, const StageParams &sp,
         overlap,
         mode == MODE_STAGE      ? dg_pack_kernel<DIM, N, MODE_STAGE, CT>
         : mode == MODE_STAGE_NC ? dg_pack_kernel<DIM, N, MODE_STAGE_NC, CT>
+        : mode == MODE_STAGE_CF ? dg_pack_kernel<DIM, N, MODE_STAGE_CF, CT>
                                 : dg_pack_kernel<DIM, N, MODE_RHS, CT>,
         (n + K::E - 1) / K::E, K::NT, K::BYTES, stream, v, n, sp, dop);
   }
@@ -106,6 +107,7 @@ cudaError_t stage_launch(const DomainView &v, int n, const StageParams &sp,
         overlap,
         mode == MODE_STAGE      ? single_kernel<DIM, N, CT, MODE_STAGE>
         : mode == MODE_STAGE_NC ? single_kernel<DIM, N, CT, MODE_STAGE_NC>
+        : mode == MODE_STAGE_CF ? single_kernel<DIM, N, CT, conforming_mode<DIM, N, CT>()>
                                 : single_kernel<DIM, N, CT, MODE_RHS>,
         grid, S::NT, smem, stream, v, n, sp, dop);
   }
@@ -145,6 +147,8 @@ template <int DIM, int N, typename CT> cudaError_t stage_prepare(int *occ)
     cudaError_t e =
         allow_smem(dg_pack_kernel<DIM, N, MODE_STAGE_NC, CT>, (int)K::BYTES);
     if (e == cudaSuccess)
+      e = allow_smem(dg_pack_kernel<DIM, N, MODE_STAGE_CF, CT>, (int)K::BYTES);
+    if (e == cudaSuccess)
       e = occupancy(dg_pack_kernel<DIM, N, MODE_STAGE, CT>, K::NT, K::BYTES,
                     &occ[MODE_STAGE]);
     if (e == cudaSuccess)
@@ -157,6 +161,9 @@ template <int DIM, int N, typename CT> cudaError_t stage_prepare(int *occ)
     using S = Shape<DIM, N>;
     const size_t smem = stage_smem_bytes<DIM, N, CT>();
     cudaError_t e = allow_smem(single_kernel<DIM, N, CT, MODE_STAGE_NC>, (int)smem);
+    if (e == cudaSuccess)
+      e = allow_smem(single_kernel<DIM, N, CT, conforming_mode<DIM, N, CT>()>,
+                     (int)smem);
     if constexpr (use_mma_hanging<DIM, N, CT>())
     {
       // as many resident CTAs in both kernels (MmaShape::MINB), so one
@@ -452,8 +459,9 @@ int launch_stage(bfam_gpu_domain_t *d, int in, double A, double B, double C,
     const int grid = d->ks.nbuf == 2 && n > slots ? (int)slots : n;
     // the first level has no coarse-side faces (unless faces glued to
     // another domain, which are lifted like them, sit there)
-    const int m = mode == MODE_STAGE && l == 0 && !d->nglued ? MODE_STAGE_NC
-                                                             : mode;
+    const int m = mode != MODE_STAGE || l > 0 || d->nglued ? mode
+                  : d->nlevels == 1                         ? MODE_STAGE_CF
+                                                            : MODE_STAGE_NC;
     bfam_gpu_domain::ProfLaunch pl{};
     if (d->prof)
     {

@@ -112,12 +112,15 @@ template <int N, typename CT = double> struct DiffOp
 // grid's operators before using it.
 
 // MODE_STAGE_NC: an LSRK stage over elements without coarse-side faces
-// (the first launch level), compiled without the coarse-face pass
+// (the first launch level), compiled without the coarse-face pass;
+// MODE_STAGE_CF: over a mesh without hanging faces, compiled without any of
+// the mortar passes
 enum
 {
   MODE_STAGE = 0,
   MODE_RHS = 1,
-  MODE_STAGE_NC = 2
+  MODE_STAGE_NC = 2,
+  MODE_STAGE_CF = 3
 };
 
 template <int DIM, int N> struct Shape

@@ -50,6 +50,7 @@
 #pragma once
 
 #include "dg_common.cuh"
+#include "dg_dmma.cuh"
 #include "dg_stage.cuh"
 
 namespace bfam_b200
@@ -98,59 +99,6 @@ template <int N> inline bool mma_for_mesh(const double *hops)
     if (bottom[i] != (i % (n + 1) == 0 ? 1.0 : 0.0))
       return true;
   return false;
-}
-
-// d += a b, one 8 x 8 x 4 step
-__device__ __forceinline__ void dmma(double2 &d, double a, double b)
-{
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 "
-               "{%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(d.x), "+d"(d.y)
-               : "d"(a), "d"(b));
-}
-
-// x[k] = Op x[k]^T for three matrices in C layout; op: Op's left fragment
-// (Op[r][2c], Op[r][2c+1])
-__device__ __forceinline__ void dmma_t3(const double2 op, double2 *x)
-{
-  double2 y[3];
-#pragma unroll
-  for (int k = 0; k < 3; ++k)
-  {
-    y[k] = make_double2(0.0, 0.0);
-    dmma(y[k], op.x, x[k].x);
-  }
-#pragma unroll
-  for (int k = 0; k < 3; ++k)
-  {
-    dmma(y[k], op.y, x[k].y);
-    x[k] = y[k];
-  }
-}
-
-// Two values of a row from p[0] and p[o1] (adjacent and 16-byte aligned if
-// VEC), and their store where they exist (v0, v1).
-template <bool VEC>
-__device__ __forceinline__ double2 get2(const double *p, int o1 = 1)
-{
-  return VEC ? *reinterpret_cast<const double2 *>(p)
-             : make_double2(p[0], p[o1]);
-}
-template <bool VEC>
-__device__ __forceinline__ void put2(double *p, const double2 x, bool v0, bool v1)
-{
-  if (VEC)
-  {
-    if (v0)
-      *reinterpret_cast<double2 *>(p) = x;
-  }
-  else
-  {
-    if (v0)
-      p[0] = x.x;
-    if (v1)
-      p[1] = x.y;
-  }
 }
 
 // L2 prefetch of what the CTA of a later work item will read of its element
@@ -408,8 +356,8 @@ __device__ __forceinline__ void mma_element(const Item &item, int n,
 #pragma unroll
       for (int q = 0; q < 6; q += 3)
       {
-        dmma_t3(oa, nb + q);
-        dmma_t3(ob, nb + q);
+        dmma_t<3>(oa, nb + q);
+        dmma_t<3>(ob, nb + q);
       }
     };
     if (hp) // coarse trace -> my piece

@@ -137,6 +137,7 @@ __device__ __forceinline__ void pack_elements(const Item &item, int n,
   const int t = threadIdx.x, first = blockIdx.x * K::E;
   const int ne = n - first < K::E ? n - first : K::E; // elements here
   const bool rd = MODE != MODE_RHS && !sp.first_stage;
+  constexpr bool HANGS = MODE != MODE_STAGE_CF; // any hanging face
 
   CT *sI = reinterpret_cast<CT *>(smem + K::OFF_IB);
   double *sP = smem + K::OFF_IB + even(Nq * Nq);
@@ -159,7 +160,7 @@ __device__ __forceinline__ void pack_elements(const Item &item, int n,
     const int es = w / NF, e = item.elem(first + es);
     const int2 ds = item.view(first + es).fdesc[(size_t)e * NF + w % NF];
     int at = -1;
-    if ((ds.y & 3) == 1 && ((ds.y >> 8) & 7) != 0)
+    if (HANGS && (ds.y & 3) == 1 && ((ds.y >> 8) & 7) != 0)
     {
       at = atomicAdd(fcount, 1);
       flist[at] = w;
@@ -243,7 +244,7 @@ __device__ __forceinline__ void pack_elements(const Item &item, int n,
     qd[c] = mine && rd ? md.dq[c * md.fs + mat] : 0.0;
   cp_async_wait<0>();
   __syncthreads();
-  const int nfine = *fcount;
+  const int nfine = HANGS ? *fcount : 0;
 
   // FP32 state minus the element's first node (see dg_stage.cuh)
   const CT *qv;
@@ -313,7 +314,7 @@ __device__ __forceinline__ void pack_elements(const Item &item, int n,
       const CT sg = (f & 1) ? CT(1) : CT(-1);
       flux_jumps<DIM, CT>(dq, f >> 1, sg, CT(ed[es].Zp), CT(ed[es].Zs),
                           fcf + 4 * (es * NF + f), sp.flux, J);
-      const int at = fidx[es * NF + f];
+      const int at = HANGS ? fidx[es * NF + f] : -1;
       if (at >= 0)
       {
         double *o = mj + at * NJ * Nfp + pn;
@@ -329,7 +330,7 @@ __device__ __forceinline__ void pack_elements(const Item &item, int n,
       for (int c = 0; c < NJ; ++c)
         put_jump<CT>(x + c * Nfp, J[jslot<DIM>(c)]);
     }
-    else if (MODE != MODE_STAGE_NC)
+    else if (MODE != MODE_STAGE_NC && HANGS)
     {
       const double *mb = d.mbuf + (size_t)ds.x * NJ * Nfp + pn;
 #pragma unroll

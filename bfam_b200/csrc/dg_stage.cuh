@@ -46,6 +46,7 @@
 #pragma once
 
 #include "dg_common.cuh"
+#include "dg_dmma.cuh"
 #include "dg_volume.cuh"
 
 namespace bfam_b200
@@ -57,6 +58,34 @@ __device__ __forceinline__ int nth_bit(int m, int i)
   for (; i > 0; --i)
     m &= m - 1;
   return __ffs(m) - 1;
+}
+
+// The mode of a launch over a mesh without hanging faces: compiled without the
+// mortar passes (N = 3 157 -> 161 and 162 -> 166 G DOF-updates/s in the two
+// forms, N = 4 137 -> 140 and 154 -> 158, 2D N = 5 138 -> 143), but for two
+// shapes that ran slower so (the plain form at N = 5 spills: 158 against 162;
+// the precision form at 2D N = 7: 171 against 174)
+template <int DIM, int N, typename CT>
+__host__ __device__ constexpr int conforming_mode()
+{
+  return (DIM == 3 && N == 5 && sizeof(CT) == sizeof(double)) ||
+                 (DIM == 2 && N == 7 && sizeof(CT) < sizeof(double))
+             ? MODE_STAGE_NC
+             : MODE_STAGE_CF;
+}
+
+// Shapes whose L2 projection (FP64) runs on the matrix instruction, a warp per
+// pair of face fields (mortar_pair): without barriers, after the node pass,
+// instead of two passes of a thread per line between barriers (3,000 of the
+// 20,800 cycles of an N = 7 element with two fine faces).  The precision form,
+// refined meshes, G DOF-updates/s before -> now: N = 7 112.7 -> 118.4, N = 6
+// 112 -> 117, N = 5 123 -> 130, N = 4 117 -> 118.5, N = 3 115.9 -> 116.8.  The
+// plain form's kernels here have no registers for it (N = 3 113 -> 110, N = 4
+// 106 -> 101).
+template <int DIM, int N, typename CT>
+__host__ __device__ constexpr bool mma_mortars()
+{
+  return DIM == 3 && N >= 3 && sizeof(CT) < sizeof(double);
 }
 
 // Node of thread t in the volume/update pass.  Nodes go in order (i
@@ -324,7 +353,7 @@ __device__ __forceinline__ void prefetch_element(const DomainView &d,
     bulk_prefetch_l2(d.fdesc + (size_t)e * NF, NF * sizeof(int2));
     bulk_prefetch_l2(d.ed + e, sizeof(ElemData));
     bulk_prefetch_l2(d.fcE + (size_t)e * NF, NF * sizeof(double4));
-    if constexpr (MODE != MODE_STAGE_NC)
+    if constexpr (MODE != MODE_STAGE_NC && MODE != MODE_STAGE_CF)
     {
       // the mortar slots of its coarse faces (written by an earlier launch)
       constexpr int NJ = S::NJ, Nfp = S::Nfp, NPC = S::NPC;
@@ -386,15 +415,22 @@ __device__ __forceinline__ void compute_element(const DomainView &d,
   const ElemData me = d.ed[e];
   const int2 *desc = d.fdesc + (size_t)e * NF;
 
-  int coarse_mask = 0, fine_mask = 0;
+  constexpr bool HANGS = MODE != MODE_STAGE_CF; // any hanging face
+  constexpr bool NO_COARSE = MODE == MODE_STAGE_NC || !HANGS;
+  int coarse_mask = 0, fine_mask = 0, pieces = 0; // 3 bits a face
 #pragma unroll
-  for (int f = 0; f < NF; ++f)
+  for (int f = 0; HANGS && f < NF; ++f)
   {
     const int y = desc[f].y;
     coarse_mask |= ((y & 3) == 2) << f;
-    fine_mask |= ((y & 3) == 1 && ((y >> 8) & 7) != 0) << f;
+    if ((y & 3) == 1 && ((y >> 8) & 7) != 0)
+    {
+      fine_mask |= 1 << f;
+      pieces |= ((y >> 8) & 7) << (3 * f);
+    }
   }
-  const int ncoarse = __popc(coarse_mask), nfine = __popc(fine_mask);
+  const int ncoarse = HANGS ? __popc(coarse_mask) : 0,
+            nfine = HANGS ? __popc(fine_mask) : 0;
 
   // ------------------------------------------------- phase 1: faces, mortars
   if (!mbar_wait(bar_q, par))
@@ -412,7 +448,7 @@ __device__ __forceinline__ void compute_element(const DomainView &d,
   // The state and flux constants come by TMA, and a thread's face pass reads
   // only its own gathered trace slots (its own cp.async group), so only the
   // fine-side interpolation, which reads whole lines, needs the barrier.
-  if (nfine)
+  if (HANGS && nfine)
     Sub<NT, EPC>::sync();
   // lift factor of face axis ax: s (2/h_ax) / w_0
   CT lfac[3];
@@ -422,6 +458,9 @@ __device__ __forceinline__ void compute_element(const DomainView &d,
         CT(s * (ax == 0 ? me.rx : (ax == 1 ? me.ry : me.rz)) * dop.iwend);
 
   // fine side: coarse partner trace -> my piece, in place (rows, then columns)
+  constexpr bool MMA = mma_mortars<DIM, N, CT>();
+  constexpr int NW = NT / 32;
+  const int wid = t >> 5;
   if (nfine)
   {
     for (int pass = 0; pass < (DIM == 3 ? 2 : 1); ++pass)
@@ -430,7 +469,7 @@ __device__ __forceinline__ void compute_element(const DomainView &d,
       {
         const int f = nth_bit(fine_mask, w / (NTF * ROWS)),
                   r = w % (NTF * ROWS);
-        const int hp = (desc[f].y >> 8) & 7;
+        const int hp = (pieces >> (3 * f)) & 7;
         const int c = r / ROWS, line = r % ROWS;
         const int half = pass == 0 ? (hp - 1) & 1 : (hp - 1) >> 1;
         const int g = f * NTF + c;
@@ -478,7 +517,7 @@ __device__ __forceinline__ void compute_element(const DomainView &d,
         const CT sg = (f & 1) ? CT(1) : CT(-1);
         flux_jumps<DIM, CT>(dq, f >> 1, sg, CT(me.Zp), CT(me.Zs),
                             fcf + 4 * f, sp.flux, J);
-        if ((fine_mask >> f) & 1)
+        if (HANGS && ((fine_mask >> f) & 1))
         {
           // rank of f among the fine faces (an element has at most DIM)
           const int fr = __popc(fine_mask & ((1 << f) - 1));
@@ -503,7 +542,7 @@ __device__ __forceinline__ void compute_element(const DomainView &d,
 
   // coarse side: the pieces' projected jumps, summed in glue order (stored
   // at the precision of the right-hand side, like the flux jumps)
-  for (int w = t; MODE != MODE_STAGE_NC && w < ncoarse * Nfp; w += NT)
+  for (int w = t; !NO_COARSE && w < ncoarse * Nfp; w += NT)
   {
     const int f = nth_bit(coarse_mask, w / Nfp), pn = w % Nfp;
     const double *mb = d.mbuf + (size_t)desc[f].x * NJ * Nfp + pn;
@@ -520,14 +559,15 @@ __device__ __forceinline__ void compute_element(const DomainView &d,
   }
 
   // fine side: L2 projection of the coarse-side jumps to the coarse face
-  // (FP64), then out to the mortar buffer for the coarse element
-  if (nfine)
+  // (FP64), then out to the mortar buffer for the coarse element (on the
+  // matrix instruction: after the node pass)
+  if (!MMA && nfine)
   {
     Sub<NT, EPC>::sync();
     for (int w = t; w < nfine * NJ * ROWS; w += NT)
     {
       const int fr = w / (NJ * ROWS), r = w % (NJ * ROWS);
-      const int hp = (desc[nth_bit(fine_mask, fr)].y >> 8) & 7;
+      const int hp = (pieces >> (3 * nth_bit(fine_mask, fr))) & 7;
       const int g = fr * NJ + r / ROWS, line = r % ROWS;
       line_apply<DIM, N, true, true, double, CT>(
           dop, (hp - 1) & 1, mj + g * Nfp, g, line);
@@ -538,7 +578,7 @@ __device__ __forceinline__ void compute_element(const DomainView &d,
       for (int w = t; w < nfine * NJ * Nq; w += NT)
       {
         const int fr = w / (NJ * Nq), r = w % (NJ * Nq);
-        const int hp = (desc[nth_bit(fine_mask, fr)].y >> 8) & 7;
+        const int hp = (pieces >> (3 * nth_bit(fine_mask, fr))) & 7;
         const int g = fr * NJ + r / Nq, col = r % Nq;
         line_apply<DIM, N, false, true, double, CT>(
             dop, (hp - 1) >> 1, mj + g * Nfp, g, col);
@@ -643,6 +683,26 @@ __device__ __forceinline__ void compute_element(const DomainView &d,
 #pragma unroll
       for (int c = 0; c < NFLD; ++c)
         d.rhs[c * fs + eoff + n] = acc[c];
+    }
+  }
+
+  // the projection, from the last warp on (at N = 7 the first warps have a
+  // second pass of nodes)
+  if constexpr (MMA && HANGS)
+  {
+    for (int w = NW - 1 - wid; w < 3 * nfine; w += NW)
+    {
+      const int fr = w / 3, c = w % 3, f = nth_bit(fine_mask, fr);
+      double2 y[2];
+      mortar_pair<N>(d.ops, 5, (pieces >> (3 * f)) & 7, mj, fr * NJ + c,
+                     fr * NJ + c + 3, y);
+      double *out =
+          d.mbuf + ((size_t)d.fslot[(size_t)e * NF + f] * NJ + c) * Nfp;
+      const int r = (t & 31) >> 2, i0 = 2 * (t & 3);
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+        put2<Nq % 2 == 0>(out + 3 * k * Nfp + i0 + Nq * r, y[k],
+                          r < Nq && i0 < Nq, r < Nq && i0 + 1 < Nq);
     }
   }
 }
