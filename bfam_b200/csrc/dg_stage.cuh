@@ -60,6 +60,30 @@ __device__ __forceinline__ int nth_bit(int m, int i)
   return __ffs(m) - 1;
 }
 
+// Two passes over face arrays of LINES lines each, arrays shared out to the
+// warps of a (sub-)element of NT threads (wid: this warp's turn), a thread per
+// line: the second pass of an array follows the first in the same warp, without
+// the other warps
+template <int LINES, int NT, typename First, typename Second>
+__device__ __forceinline__ void for_arrays(int wid, int arrays,
+                                           const First &first,
+                                           const Second &second)
+{
+  constexpr int PER = 32 / LINES; // arrays per warp
+  const int lane = threadIdx.x & 31;
+  for (int a0 = wid * PER; a0 < arrays; a0 += NT / 32 * PER)
+  {
+    const int a = a0 + lane / LINES, line = lane % LINES;
+    const bool mine = lane < PER * LINES && a < arrays;
+    if (mine)
+      first(a, line);
+    __syncwarp();
+    if (mine)
+      second(a, line);
+    __syncwarp();
+  }
+}
+
 // The mode of a launch over a mesh without hanging faces: compiled without the
 // mortar passes (N = 3 157 -> 161 and 162 -> 166 G DOF-updates/s in the two
 // forms, N = 4 137 -> 140 and 154 -> 158, 2D N = 5 138 -> 143), but for two
@@ -74,14 +98,17 @@ __host__ __device__ constexpr int conforming_mode()
              : MODE_STAGE_CF;
 }
 
-// Shapes whose L2 projection (FP64) runs on the matrix instruction, a warp per
-// pair of face fields (mortar_pair): without barriers, after the node pass,
-// instead of two passes of a thread per line between barriers (3,000 of the
-// 20,800 cycles of an N = 7 element with two fine faces).  The precision form,
-// refined meshes, G DOF-updates/s before -> now: N = 7 112.7 -> 118.4, N = 6
-// 112 -> 117, N = 5 123 -> 130, N = 4 117 -> 118.5, N = 3 115.9 -> 116.8.  The
-// plain form's kernels here have no registers for it (N = 3 113 -> 110, N = 4
-// 106 -> 101).
+// Shapes (the precision form in 3D) whose mortar passes stay within a warp: the
+// interpolation's two passes over an array by the same warp (for_arrays, one
+// barrier instead of two), and the L2 projection (FP64) on the matrix
+// instruction, a warp per pair of face fields (mortar_pair), without barriers
+// and after the node pass.  A thread per line between CTA barriers took 3,700
+// and 3,000 of the 20,800 cycles of an N = 7 element with two fine faces.
+// Refined meshes, G DOF-updates/s before -> with the projection -> with both:
+// N = 7 112.7 -> 118.4 -> 121.3, N = 6 112 -> 117 -> 118, N = 5 123 -> 130.1 ->
+// 130.4, N = 4 117 -> 118.5 -> 119.3, N = 3 115.9 -> 117.0 -> 117.9.  The plain
+// form's kernels here have no registers for it (N = 3 114 -> 110, N = 4 107 ->
+// 101).
 template <int DIM, int N, typename CT>
 __host__ __device__ constexpr bool mma_mortars()
 {
@@ -463,23 +490,40 @@ __device__ __forceinline__ void compute_element(const DomainView &d,
   const int wid = t >> 5;
   if (nfine)
   {
-    for (int pass = 0; pass < (DIM == 3 ? 2 : 1); ++pass)
+    if constexpr (MMA)
     {
-      for (int w = t; w < nfine * NTF * ROWS; w += NT)
-      {
-        const int f = nth_bit(fine_mask, w / (NTF * ROWS)),
-                  r = w % (NTF * ROWS);
+      // an array's rows, then its columns, by the same warp
+      for_arrays<Nq, NT>(wid, nfine * NTF, [&](int a, int line) {
+        const int f = nth_bit(fine_mask, a / NTF), g = f * NTF + a % NTF;
         const int hp = (pieces >> (3 * f)) & 7;
-        const int c = r / ROWS, line = r % ROWS;
-        const int half = pass == 0 ? (hp - 1) & 1 : (hp - 1) >> 1;
-        const int g = f * NTF + c;
-        if (pass == 0)
-          line_apply<DIM, N, true, false, CT, CT>(dop, half, pt + g * Nfp, g, line);
-        else
-          line_apply<DIM, N, false, false, CT, CT>(dop, half, pt + g * Nfp, g, line);
-      }
+        line_apply<DIM, N, true, false, CT, CT>(dop, (hp - 1) & 1, pt + g * Nfp,
+                                                g, line);
+      }, [&](int a, int line) {
+        const int f = nth_bit(fine_mask, a / NTF), g = f * NTF + a % NTF;
+        const int hp = (pieces >> (3 * f)) & 7;
+        line_apply<DIM, N, false, false, CT, CT>(dop, (hp - 1) >> 1,
+                                                 pt + g * Nfp, g, line);
+      });
       Sub<NT, EPC>::sync();
     }
+    else
+      for (int pass = 0; pass < (DIM == 3 ? 2 : 1); ++pass)
+      {
+        for (int w = t; w < nfine * NTF * ROWS; w += NT)
+        {
+          const int f = nth_bit(fine_mask, w / (NTF * ROWS)),
+                    r = w % (NTF * ROWS);
+          const int hp = (pieces >> (3 * f)) & 7;
+          const int c = r / ROWS, line = r % ROWS;
+          const int half = pass == 0 ? (hp - 1) & 1 : (hp - 1) >> 1;
+          const int g = f * NTF + c;
+          if (pass == 0)
+            line_apply<DIM, N, true, false, CT, CT>(dop, half, pt + g * Nfp, g, line);
+          else
+            line_apply<DIM, N, false, false, CT, CT>(dop, half, pt + g * Nfp, g, line);
+        }
+        Sub<NT, EPC>::sync();
+      }
   }
 
   // flux on conforming and fine-side faces: the face node's jumps (T* - T-,
@@ -686,9 +730,11 @@ __device__ __forceinline__ void compute_element(const DomainView &d,
     }
   }
 
-  // the projection, from the last warp on (at N = 7 the first warps have a
-  // second pass of nodes)
-  if constexpr (MMA && HANGS)
+  // Fine side: L2 projection of the coarse-side jumps to the coarse face
+  // (FP64) and their store to the mortar buffer for the coarse element, after
+  // the node pass and from the last warp on (at N = 7 the first warps have a
+  // second pass of nodes): no other warp waits for it
+  if constexpr (HANGS && MMA)
   {
     for (int w = NW - 1 - wid; w < 3 * nfine; w += NW)
     {
