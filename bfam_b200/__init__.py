@@ -631,7 +631,7 @@ def tile_elements(dim: int, N: int) -> list[int]:
 
 
 class Batch:
-    """bfam_gpu_batch_t: domains stepped together, one persistent launch per
+    """bfam_gpu_batch_t: domains stepped together, one launch per
     order group and stage."""
 
     def __init__(self, domains, method: int = LSRK_KC54, t0=None):

@@ -3,9 +3,8 @@
 A batch runs one launch per order group, level and LSRK stage.  The tile of a
 group is (elements per CTA, threads per element, register budget for a
 number of resident CTAs per SM), chosen among the shapes compiled for that
-order (`tile_shapes`, `tile_elements`), plus the CTAs per SM of a persistent
-grid (two-buffer tiles) or of the L2 lookahead distance (one-buffer tiles).  The tuner times
-every candidate on a synthetic domain of the group's order, precision and
+order (`tile_shapes`, `tile_elements`), plus the CTAs per SM of the L2
+lookahead distance.  The tuner times every candidate on a synthetic domain of the group's order, precision and
 roughly its element count (a 20 % refined brick, Gaussian pulse, random
 material, capped in size so tuning takes seconds), with CUDA events on the
 batch's stream over a few graph-replayed steps, and keeps the fastest.

@@ -5,7 +5,7 @@
 // Each group owns a flat work list of (domain, element) pairs, domain-major,
 // and per state parity an array of the stage kernel's domain views (state
 // buffers, time step, source, clock of each domain).  One LSRK stage is one
-// persistent launch per group; groups run on streams forked from the
+// launch per group and refinement level; groups run on streams forked from the
 // batch's stream, and the step ends with one post-step launch over all
 // domains (receivers, clocks).  A step is captured once per parity into a
 // CUDA graph and replayed.
@@ -40,7 +40,8 @@ typedef int (*batch_occupancy_fn)();
 
 struct BatchTile
 {
-  int NT = 0, MINB = 0, NBUF = 1;
+  int NT = 0, MINB = 0;
+  int lookahead = 2; // L2 lookahead: that part of a wave of resident CTAs
   int EPC = 1; // elements per CTA (NT threads each)
   int pack = 0; // elements per CTA of the packed kernel (0: not packed)
   batch_launch_fn launch = nullptr;
@@ -63,10 +64,9 @@ struct BatchTile
 template <int DIM, int N, int NT, int MINB, typename CT, int EPC = 1>
 struct TileImpl
 {
-  static constexpr int NB = EPC == 1 ? nbuf<DIM, N, CT>() : 1;
   template <int MODE>
   static constexpr auto kernel =
-      dg_stage_batch_kernel<DIM, N, NT, MINB, MODE, CT, NB, EPC>;
+      dg_stage_batch_kernel<DIM, N, NT, MINB, MODE, CT, EPC>;
   static constexpr size_t SMEM = stage_smem_bytes<DIM, N, CT, EPC>();
   template <int MODE>
   static cudaError_t run(const DomainView *v, const int2 *w, int nwork,
@@ -107,7 +107,6 @@ struct TileImpl
     t.NT = NT;
     t.MINB = MINB;
     t.EPC = EPC;
-    t.NBUF = NB;
     t.launch = run<MODE_STAGE>;
     t.launch_nc = run<MODE_STAGE_NC>;
     t.launch_cf = run<conforming_mode<DIM, N, CT>()>;
@@ -217,6 +216,7 @@ template <int N, int MINB> struct MmaTile
     BatchTile t;
     t.NT = M::NT;
     t.MINB = MINB;
+    t.lookahead = N == 7 ? 4 : 2; // as for single domains
     t.launch = t.launch_nc = t.launch_cf = launch;
     t.prepare = prepare;
     t.occupancy = occupancy;
@@ -561,17 +561,12 @@ int choose_grid(bfam_gpu_batch_t *b, bfam_gpu_batch_t::Group &g)
   const int per_sm = g.ctas_per_sm > 0 && g.ctas_per_sm < occ ? g.ctas_per_sm
                                                                : occ;
   const int64_t full = (int64_t)per_sm * b->sms;
-  // a persistent grid for two-buffer tiles; one CTA per work item for
-  // one-buffer tiles
-  const bool persistent = t.NBUF == 2;
-  // L2 lookahead in work items: half a wave of resident elements
+  // L2 lookahead in work items
   const int epc = t.pack ? t.pack : t.EPC;
-  g.ahead = persistent ? 0
-                       : (int)std::min<int64_t>(full * epc / 2, INT32_MAX);
+  g.ahead = (int)std::min<int64_t>(full * epc / t.lookahead, INT32_MAX);
   g.grid.resize(g.nwork_l.size());
   for (size_t l = 0; l < g.nwork_l.size(); ++l)
-    g.grid[l] = (int)(persistent ? (g.nwork_l[l] > full ? full : g.nwork_l[l])
-                                 : (g.nwork_l[l] + t.EPC - 1) / t.EPC);
+    g.grid[l] = (int)((g.nwork_l[l] + t.EPC - 1) / t.EPC);
   return 0;
 }
 
@@ -645,7 +640,7 @@ int launch_level(bfam_gpu_batch_t *b, bfam_gpu_batch::Group &g, size_t l,
     if (d->nlevels > 1)
       v.elist = d->elist + d->level_off[l];
     CUDA_TRY(d->ks.launch(v, (int)g.nwork_l[l], sp, g.hops.data(),
-                          mode, g.grid[l], st, overlap));
+                          mode, st, overlap));
     return 0;
   }
   const BatchTile &t = g.tiles[g.tile];

@@ -55,7 +55,7 @@ namespace
 template <int DIM, int N, typename CT, int MODE>
 constexpr auto single_kernel =
     dg_stage_kernel<DIM, N, Shape<DIM, N>::NT, stage_min_ctas<DIM, N, CT>(),
-                    MODE, CT, nbuf<DIM, N, CT>()>;
+                    MODE, CT>;
 
 template <int N, int MODE>
 constexpr auto mma_kernel = dg_mma_kernel<N, MmaShape<N>::MINB, MODE>;
@@ -73,11 +73,11 @@ cudaError_t mma_launch(const DomainView &v, int n, const StageParams &sp,
                           1.0 / hops[7 * (N + 1) * (N + 1)]);
 }
 
-// n work items on a persistent grid of `grid` CTAs
+// n work items, a CTA for each element (packed: for several)
 template <int DIM, int N, typename CT>
 cudaError_t stage_launch(const DomainView &v, int n, const StageParams &sp,
-                         const double *hops, int mode, int grid,
-                         cudaStream_t stream, bool overlap)
+                         const double *hops, int mode, cudaStream_t stream,
+                         bool overlap)
 {
   if constexpr (use_mma_hanging<DIM, N, CT>())
   {
@@ -109,7 +109,7 @@ cudaError_t stage_launch(const DomainView &v, int n, const StageParams &sp,
         : mode == MODE_STAGE_NC ? single_kernel<DIM, N, CT, MODE_STAGE_NC>
         : mode == MODE_STAGE_CF ? single_kernel<DIM, N, CT, conforming_mode<DIM, N, CT>()>
                                 : single_kernel<DIM, N, CT, MODE_RHS>,
-        grid, S::NT, smem, stream, v, n, sp, dop);
+        n, S::NT, smem, stream, v, n, sp, dop);
   }
 }
 
@@ -191,11 +191,10 @@ template <int DIM, int N, typename CT> KernelSet make_set()
   k.prepare = stage_prepare<DIM, N, CT>;
   k.energy = dg_energy_kernel<DIM, N>;
   k.NT = S::NT;
+  if (use_mma<DIM, N, CT>() && N == 7)
+    k.lookahead = 4; // 157 against 155.6 G DOF-updates/s on refined meshes
   if (use_pack<DIM, N, CT>())
     k.elements = PackShape<DIM, N, CT>::E;
-  k.nbuf = use_mma<DIM, N, CT>() || use_pack<DIM, N, CT>()
-               ? 1
-               : nbuf<DIM, N, CT>();
   return k;
 }
 
@@ -434,11 +433,9 @@ int launch_stage(bfam_gpu_domain_t *d, int in, double A, double B, double C,
   sp.C = C;
   sp.first_stage = first;
   sp.flux = d->flux;
-  // one element per CTA: prefetch half a wave of resident CTAs ahead (about
-  // half a CTA lifetime before the element's CTA starts)
-  sp.ahead = d->ks.nbuf == 1
-                 ? d->ks.occ[mode] * d->sms * d->ks.elements / 2
-                 : 0;
+  // prefetch part of a wave of resident CTAs ahead (half a wave: about half a
+  // CTA lifetime before the element's CTA starts)
+  sp.ahead = d->ks.occ[mode] * d->sms * d->ks.elements / d->ks.lookahead;
   DomainView v = view(d, in);
   v.dt = dt;
   // one launch per level; level l's elements after level l-1's
@@ -452,11 +449,6 @@ int launch_stage(bfam_gpu_domain_t *d, int in, double A, double B, double C,
     }
     if (n == 0)
       continue;
-    // two element buffers: a persistent grid (every resident CTA slot)
-    // whose CTAs overlap the next element's loads with the current one; one
-    // buffer: one CTA per element, balanced by the block scheduler
-    const int64_t slots = (int64_t)d->ks.occ[mode] * d->sms;
-    const int grid = d->ks.nbuf == 2 && n > slots ? (int)slots : n;
     // the first level has no coarse-side faces (unless faces glued to
     // another domain, which are lifted like them, sit there)
     const int m = mode != MODE_STAGE || l > 0 || d->nglued ? mode
@@ -483,7 +475,7 @@ int launch_stage(bfam_gpu_domain_t *d, int in, double A, double B, double C,
       pl.bytes = per_dof * (double)n * d->Np * d->NFLD;
       CUDA_TRY(cudaEventRecord(pl.t0, d->stream));
     }
-    CUDA_TRY(d->ks.launch(v, n, sp, d->hops.data(), m, grid, d->stream,
+    CUDA_TRY(d->ks.launch(v, n, sp, d->hops.data(), m, d->stream,
                            true));
     g_launches.fetch_add(1, std::memory_order_relaxed);
     if (d->prof)

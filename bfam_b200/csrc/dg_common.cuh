@@ -159,8 +159,8 @@ template <int DIM, int N> struct Shape
   //     106 refined; four 128 and 94, seven 132 and 100, eight 134 and 104),
   //     seven in the precision form (156 and 117; four 134 and 96, six 143
   //     and 104, eight 134 and 101);
-  //   3D N=6, precision form: three CTAs of 352 threads with one buffer (141
-  //     and 112; two CTAs 129 and 98, one with two buffers 106 and 74);
+  //   3D N=6, precision form: three CTAs of 352 threads (141 and 112; two
+  //     129 and 98, one 106 and 74);
   //   3D N=7, precision form: two CTAs of 384 threads (three: 92.2 vs 102.3,
   //     spills).
   static constexpr int MINB_RAW = 65536 / (NT * 96);

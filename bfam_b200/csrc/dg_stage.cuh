@@ -150,12 +150,10 @@ template <typename CT> __device__ __forceinline__ CT get_jump(const double *slot
 }
 
 // Shared-memory layout of one CTA (in doubles, every region 16-byte
-// aligned).  NBUF element buffers (state, dq, face traces / flux jumps, face
-// flux constants) let the loads of the next element fly
-// while the current one is computed; the mortar scratch, the differentiation
-// matrix, the mbarriers (q and dq per buffer) and the precision form's FP32 tile are
-// single.
-template <int DIM, int N, typename CT, int NBUF, bool DQS = true> struct Tile
+// aligned): state, dq where it is staged, face traces / flux jumps, face flux
+// constants, the mortar scratch, the differentiation matrix, the mbarriers (q
+// and dq) and the precision form's FP32 tile.
+template <int DIM, int N, typename CT, bool DQS = true> struct Tile
 {
   using S = Shape<DIM, N>;
   // DQS: the element's dq rows are staged in shared memory (TMA); otherwise
@@ -164,10 +162,10 @@ template <int DIM, int N, typename CT, int NBUF, bool DQS = true> struct Tile
   // cost 1-2 % at N = 5 and 7)
   static constexpr int BUF =
       S::SM_QS + (DQS ? S::SM_DQ : 0) + S::SM_PT + 4 * S::NF;
-  static constexpr int OFF_MJ = NBUF * BUF;
+  static constexpr int OFF_MJ = BUF;
   static constexpr int OFF_OPS = OFF_MJ + S::SM_MJ;
   static constexpr int OFF_BAR = OFF_OPS + S::SM_IP;
-  static constexpr int OFF_QV = OFF_BAR + 2 * NBUF;
+  static constexpr int OFF_QV = OFF_BAR + 2;
   static constexpr bool NARROW = sizeof(CT) < sizeof(double);
   static constexpr int TOTAL = OFF_QV + (NARROW ? S::SM_QF : 0);
   static constexpr size_t BYTES = (size_t)TOTAL * sizeof(double);
@@ -180,12 +178,12 @@ template <int DIM, int N, typename CT> __host__ __device__ constexpr int shape_m
                                      : Shape<DIM, N>::MINB;
 }
 
-// CTAs per SM that the shape's register budget and NBUF buffers admit
+// CTAs per SM that the shape's register budget and shared memory admit
 // (228 KB of shared memory per SM, 1 KB reserved per CTA)
-template <int DIM, int N, typename CT, int NBUF, bool DQS = true>
+template <int DIM, int N, typename CT, bool DQS = true>
 __host__ __device__ constexpr int resident_ctas()
 {
-  constexpr size_t bytes = Tile<DIM, N, CT, NBUF, DQS>::BYTES;
+  constexpr size_t bytes = Tile<DIM, N, CT, DQS>::BYTES;
   constexpr int by_smem = bytes > 227 * 1024 ? 0 : (int)(233472 / (bytes + 1024));
   constexpr int m = shape_minb<DIM, N, CT>();
   return m < by_smem ? m : by_smem;
@@ -200,25 +198,8 @@ template <int DIM, int N, typename CT> __host__ __device__ constexpr bool stage_
   if (Shape<DIM, N>::DQ_L2 ||
       (Shape<DIM, N>::DQ_L2_NARROW && sizeof(CT) < sizeof(double)))
     return false;
-  return resident_ctas<DIM, N, CT, 1, true>() >=
-         resident_ctas<DIM, N, CT, 1, false>();
-}
-
-// Two buffers (a persistent grid; the loads of the next element overlap the
-// current one) only where one buffer leaves fewer than four resident CTAs
-// per SM and the second buffer costs none.  With four or more one-element
-// CTAs per SM the block scheduler's balancing of the uneven element costs
-// wins (3D N=3: 105.8 vs 91.5 G DOF-updates/s, N=4: 83.7 vs 72.0, 2D N=3:
-// 54.0 vs 51.3; 3D N=2: 57.5 vs 61.0 in FP64 but 66.6 vs 59.2 in the
-// precision form; 2D N=5: 61.8 vs 70.5), and a second buffer that costs
-// resident CTAs loses (N=5: three CTAs of 7 warps with one buffer, two with
-// two).
-template <int DIM, int N, typename CT> __host__ __device__ constexpr int nbuf()
-{
-  constexpr bool DQS = stage_dqs<DIM, N, CT>();
-  constexpr int one = resident_ctas<DIM, N, CT, 1, DQS>(),
-                two = resident_ctas<DIM, N, CT, 2, DQS>();
-  return one < 4 && two >= one && two > 0 ? 2 : 1;
+  return resident_ctas<DIM, N, CT, true>() >=
+         resident_ctas<DIM, N, CT, false>();
 }
 
 // Elements per CTA: a CTA of EPC * NT threads holds EPC sub-elements of NT
@@ -258,41 +239,40 @@ __device__ __forceinline__ double *sub_smem()
   return EPC == 1 ? smem : smem + Sub<NT, EPC>::id() * T::TOTAL;
 }
 
-// Element buffer b of the tile.
-template <int DIM, int N, typename CT, int NBUF, int NT = 32, int EPC = 1>
+// The element's buffer in the tile.
+template <int DIM, int N, typename CT, int NT = 32, int EPC = 1>
 struct TileBuf
 {
   double *qs, *R, *pt, *fcf;
   uint64_t *bq, *bdq;
-  __device__ __forceinline__ explicit TileBuf(int b)
+  __device__ __forceinline__ TileBuf()
   {
     using S = Shape<DIM, N>;
     constexpr bool DQS = stage_dqs<DIM, N, CT>();
-    using T = Tile<DIM, N, CT, NBUF, DQS>;
+    using T = Tile<DIM, N, CT, DQS>;
     double *smem = sub_smem<T, NT, EPC>();
-    qs = smem + b * T::BUF;
+    qs = smem;
     R = qs + S::SM_QS;
     pt = R + (DQS ? S::SM_DQ : 0);
     fcf = pt + S::SM_PT;
-    bq = reinterpret_cast<uint64_t *>(smem + T::OFF_BAR) + 2 * b;
+    bq = reinterpret_cast<uint64_t *>(smem + T::OFF_BAR);
     bdq = bq + 1;
   }
 };
 
-// Issue every global read of element e into buffer b: q and (after the first
-// stage) dq by TMA bulk copies completing on the buffer's mbarriers, the
-// neighbours' face traces and the face flux constants by cp.async, as one
-// commit group.
-template <int DIM, int N, int NT, int MODE, typename CT, int NBUF,
-          int EPC = 1>
+// Issue every global read of element e: q and (after the first stage, where it
+// is staged) dq by TMA bulk copies completing on the mbarriers, the
+// neighbours' face traces by cp.async, as one commit group.  ds0: descriptor
+// of the face of thread t's first face node.
+template <int DIM, int N, int NT, int MODE, typename CT, int EPC = 1>
 __device__ __forceinline__ void issue_element(const DomainView &d,
                                               const StageParams &sp, int e,
-                                              int b)
+                                              int2 ds0)
 {
   using S = Shape<DIM, N>;
   constexpr int Np = S::Np, Nfp = S::Nfp, NF = S::NF, NFLD = S::NFLD,
                 NTF = S::NTF, PITCH = S::PITCH;
-  const TileBuf<DIM, N, CT, NBUF, NT, EPC> tb(b);
+  const TileBuf<DIM, N, CT, NT, EPC> tb;
   double *qs = tb.qs, *R = tb.R, *pt = tb.pt, *fcf = tb.fcf;
   uint64_t *bar_q = tb.bq, *bar_dq = tb.bdq;
   const int t = Sub<NT, EPC>::t();
@@ -332,7 +312,7 @@ __device__ __forceinline__ void issue_element(const DomainView &d,
   for (int w = t; w < NF * Nfp; w += NT)
   {
     const int f = w / Nfp, pn = w % Nfp;
-    const int2 ds = desc[f];
+    const int2 ds = NF * Nfp <= NT || w == t ? ds0 : desc[f];
     const int k = ds.y & 3;
     if (k == 2)
       continue;
@@ -396,17 +376,15 @@ __device__ __forceinline__ void prefetch_element(const DomainView &d,
   }
 }
 
-// Compute element e from buffer b (its loads issued by issue_element; `par`
-// is the buffer's mbarrier phase parity).
-template <int DIM, int N, int NT, int MODE, typename CT, int NBUF,
-          int EPC = 1>
+// Compute element e, its loads issued by issue_element.
+template <int DIM, int N, int NT, int MODE, typename CT, int EPC = 1>
 __device__ __forceinline__ void compute_element(const DomainView &d,
                                                 const StageParams &sp,
                                                 const DiffOp<N, CT> &dop,
-                                                int e, int b, unsigned par)
+                                                int e)
 {
   using S = Shape<DIM, N>;
-  using T = Tile<DIM, N, CT, NBUF, stage_dqs<DIM, N, CT>()>;
+  using T = Tile<DIM, N, CT, stage_dqs<DIM, N, CT>()>;
   constexpr int Nq = S::Nq, Np = S::Np, Nfp = S::Nfp, NF = S::NF,
                 NFLD = S::NFLD, NJ = S::NJ, NPC = S::NPC, ROWS = S::ROWS,
                 NTF = S::NTF, PITCH = S::PITCH;
@@ -414,7 +392,7 @@ __device__ __forceinline__ void compute_element(const DomainView &d,
   // (not a pointer parameter), so that all accesses stay in the shared
   // window with 32-bit addressing
   double *smem = sub_smem<T, NT, EPC>();
-  const TileBuf<DIM, N, CT, NBUF, NT, EPC> tb(b);
+  const TileBuf<DIM, N, CT, NT, EPC> tb;
   double *qs = tb.qs, *pt = tb.pt, *fcf = tb.fcf;
   uint64_t *bar_q = tb.bq, *bar_dq = tb.bdq;
   // field rows of the state and of dq
@@ -460,9 +438,9 @@ __device__ __forceinline__ void compute_element(const DomainView &d,
             nfine = HANGS ? __popc(fine_mask) : 0;
 
   // ------------------------------------------------- phase 1: faces, mortars
-  if (!mbar_wait(bar_q, par))
+  if (!mbar_wait(bar_q, 0))
     atomicExch(d.err, 1);
-  cp_async_wait<NBUF - 1>(); // this element's group (the next one may fly)
+  cp_async_wait<0>();
   if constexpr (NARROW)
   {
     for (int n = t; n < Np; n += NT)
@@ -648,7 +626,7 @@ __device__ __forceinline__ void compute_element(const DomainView &d,
   constexpr bool DQS = stage_dqs<DIM, N, CT>();
   if (MODE != MODE_RHS && rd && DQS)
   {
-    if (!mbar_wait(bar_dq, par))
+    if (!mbar_wait(bar_dq, 0))
       atomicExch(d.err, 2);
   }
   constexpr int NODE_ITERS = (Np + NT - 1) / NT;
@@ -755,27 +733,24 @@ __device__ __forceinline__ void compute_element(const DomainView &d,
 
 
 // The launch's work items: item.view(idx) and item.elem(idx) give item idx's
-// domain view and element.  With one buffer every CTA does one item (the
-// grid covers them all); with two buffers the grid is persistent (items
-// blockIdx.x, blockIdx.x + gridDim.x, ...) and the loads of the next item
-// are issued before the current one is computed.
-template <int DIM, int N, int NT, int MODE, typename CT, int NBUF,
-          typename Item, int EPC = 1>
+// domain view and element; a CTA does one item (EPC of them), and the block
+// scheduler balances the uneven element costs.
+template <int DIM, int N, int NT, int MODE, typename CT, typename Item,
+          int EPC = 1>
 __device__ __forceinline__ void stage_loop(const Item &item, int n,
                                            const StageParams &sp,
                                            const DiffOp<N, CT> &dop)
 {
-  using T = Tile<DIM, N, CT, NBUF, stage_dqs<DIM, N, CT>()>;
+  using T = Tile<DIM, N, CT, stage_dqs<DIM, N, CT>()>;
   using SB = Sub<NT, EPC>;
-  static_assert(EPC == 1 || NBUF == 1, "sub-elements use one buffer each");
   constexpr int Nq = N + 1;
   double *smem = sub_smem<T, NT, EPC>();
   const int lt = SB::t();
   if (lt == 0)
   {
     uint64_t *bar = reinterpret_cast<uint64_t *>(smem + T::OFF_BAR);
-    for (int i = 0; i < 2 * NBUF; ++i)
-      mbar_init(&bar[i], 1);
+    mbar_init(&bar[0], 1);
+    mbar_init(&bar[1], 1);
   }
   // the differentiation matrix into shared memory (rows indexed per
   // thread in the volume pass; the mortar operators are read from the
@@ -786,42 +761,26 @@ __device__ __forceinline__ void stage_loop(const Item &item, int n,
       sD[w] = dop.D[w];
   }
   SB::sync();
-  int idx = (int)blockIdx.x * EPC + SB::id();
-  grid_dependency_wait(); // the stage input is complete
+  // one element per sub-element (the grid covers every item)
+  const int idx = (int)blockIdx.x * EPC + SB::id();
   if (idx >= n)
     return;
-  if constexpr (NBUF == 1)
-  {
-    // one element per sub-element (the grid covers every item)
-    issue_element<DIM, N, NT, MODE, CT, 1, EPC>(item.view(idx), sp,
-                                                item.elem(idx), 0);
-    // a thread of another warp than the TMA issuer prefetches a later
-    // item's element while this one's loads fly
-    const int ia = idx + sp.ahead;
-    if (sp.ahead > 0 && ia < n && lt == (NT > 32 ? 32 : 0))
-      prefetch_element<DIM, N, MODE>(item.view(ia), sp, item.elem(ia));
-    compute_element<DIM, N, NT, MODE, CT, 1, EPC>(item.view(idx), sp, dop,
-                                                  item.elem(idx), 0, 0);
-    return;
-  }
-  issue_element<DIM, N, NT, MODE, CT, NBUF>(item.view(idx), sp,
-                                            item.elem(idx), 0);
-#pragma unroll 1
-  for (unsigned it = 0; idx < n; ++it)
-  {
-    const int b = (int)(it & 1u);
-    const unsigned par = (it >> 1) & 1u;
-    const int nidx = idx + (int)gridDim.x;
-    if (nidx < n)
-      issue_element<DIM, N, NT, MODE, CT, NBUF>(item.view(nidx), sp,
-                                                item.elem(nidx), b ^ 1);
-    else
-      cp_async_commit(); // keep one group per iteration
-    compute_element<DIM, N, NT, MODE, CT, NBUF>(item.view(idx), sp, dop,
-                                                item.elem(idx), b, par);
-    __syncthreads(); // buffer b is free
-    idx = nidx;
-  }
+  // the tables are constant: the element and the descriptor of this thread's
+  // first face node are read while the launch before still runs (two trips to
+  // memory per launch: 3D N = 3 on 211 elements 48.3 -> 44.2 us per step, N = 7
+  // 99 -> 94; refined 30 M DOF meshes +1 %)
+  constexpr int NF = Shape<DIM, N>::NF, Nfp = Shape<DIM, N>::Nfp;
+  const DomainView &d = item.view(idx);
+  const int e = item.elem(idx), f0 = lt / Nfp;
+  const int2 ds0 = d.fdesc[(size_t)e * NF + (f0 < NF ? f0 : NF - 1)];
+  grid_dependency_wait(); // the stage input is complete
+  issue_element<DIM, N, NT, MODE, CT, EPC>(d, sp, e, ds0);
+  // a thread of another warp than the TMA issuer prefetches a later
+  // item's element while this one's loads fly
+  const int ia = idx + sp.ahead;
+  if (sp.ahead > 0 && ia < n && lt == (NT > 32 ? 32 : 0))
+    prefetch_element<DIM, N, MODE>(item.view(ia), sp, item.elem(ia));
+  compute_element<DIM, N, NT, MODE, CT, EPC>(d, sp, dop, e);
 }
 
 // one domain: item idx is element idx, or the idx-th of an element list
@@ -859,18 +818,18 @@ struct BatchItems
 
 // One domain: item idx is element idx, or the idx-th of the launch's
 // element list (meshes with hanging faces launch their elements by level).
-template <int DIM, int N, int NT, int MINB, int MODE, typename CT, int NBUF>
+template <int DIM, int N, int NT, int MINB, int MODE, typename CT>
 __global__ void __launch_bounds__(NT, MINB)
     dg_stage_kernel(DomainView d, int n, StageParams sp,
                     const __grid_constant__ DiffOp<N, CT> dop)
 {
-  stage_loop<DIM, N, NT, MODE, CT, NBUF>(SingleItems{d}, n, sp, dop);
+  stage_loop<DIM, N, NT, MODE, CT>(SingleItems{d}, n, sp, dop);
 }
 
 // Many domains of the same order: item idx is work[idx] = (domain, element),
 // each domain with its own arrays and time step.  EPC elements per CTA of
-// EPC * NT threads (one buffer each).
-template <int DIM, int N, int NT, int MINB, int MODE, typename CT, int NBUF,
+// EPC * NT threads.
+template <int DIM, int N, int NT, int MINB, int MODE, typename CT,
           int EPC = 1>
 __global__ void __launch_bounds__(NT *EPC, MINB)
     dg_stage_batch_kernel(const DomainView *__restrict__ views,
@@ -878,18 +837,15 @@ __global__ void __launch_bounds__(NT *EPC, MINB)
                           StageParams sp,
                           const __grid_constant__ DiffOp<N, CT> dop)
 {
-  stage_loop<DIM, N, NT, MODE, CT, NBUF, BatchItems, EPC>(
+  stage_loop<DIM, N, NT, MODE, CT, BatchItems, EPC>(
       BatchItems{views, work}, nwork, sp, dop);
 }
 
-// dynamic shared memory of one CTA of the stage kernels (EPC sub-elements of
-// one buffer each when EPC > 1)
+// dynamic shared memory of one CTA of the stage kernels (EPC sub-elements)
 template <int DIM, int N, typename CT, int EPC = 1>
 __host__ __device__ constexpr size_t stage_smem_bytes()
 {
-  return EPC == 1
-             ? Tile<DIM, N, CT, nbuf<DIM, N, CT>(), stage_dqs<DIM, N, CT>()>::BYTES
-             : EPC * Tile<DIM, N, CT, 1, stage_dqs<DIM, N, CT>()>::BYTES;
+  return EPC * Tile<DIM, N, CT, stage_dqs<DIM, N, CT>()>::BYTES;
 }
 
 // resident CTAs per SM the register budget is sized for: the shape's choice,

@@ -58,8 +58,7 @@ cudaError_t launch_dependent(bool overlap, void (*kernel)(P...), dim3 grid,
 // per-order launchers (the kernels' parameter lists depend on the order)
 typedef cudaError_t (*stage_launch_fn)(const DomainView &, int n,
                                 const StageParams &, const double *D,
-                                int mode, int grid, cudaStream_t,
-                                bool overlap);
+                                int mode, cudaStream_t, bool overlap);
 typedef cudaError_t (*prepare_fn)(int *occ);
 typedef void (*energy_fn)(const double *, size_t, const ElemData *,
                           const double *, double *);
@@ -71,8 +70,8 @@ struct KernelSet
   energy_fn energy = nullptr;
   int NT = 0;
   int occ[2] = {0, 0}; // resident CTAs per SM of the stage and rhs kernels
-  int nbuf = 1;        // element buffers per CTA
   int elements = 1;    // elements per CTA
+  int lookahead = 2;   // L2 lookahead: that part of a wave of resident CTAs
 };
 
 // the kernels of one (dim, order, precision)

@@ -10,7 +10,7 @@ runs continuous batching:
     their host-side setup (mesh, tables, upload) overlaps the GPU work in
     flight;
   * the active set advances in chunks of steps: one bfam_gpu_batch_step of
-    `chunk` steps (persistent launches per order group, graph-replayed),
+    `chunk` steps (launches per order group and stage, graph-replayed),
     never past the end of the shortest remaining request;
   * between chunks finished requests are retired (seismograms downloaded,
     device memory returned to the pool) and the requests admitted during

@@ -350,8 +350,9 @@ int bfam_gpu_domain_get_seismograms(bfam_gpu_domain_t *dom, double *out,
 /* ------------------------------------------------------------------------
  * Batches: many independent domains stepped together.  No counterpart in
  * the reference (one bfam domain per MPI rank).  Domains are grouped by
- * (dim, order, precision, flux, operators); each group is one persistent
- * launch per LSRK stage over a flat (domain, element) work list, the groups
+ * (dim, order, precision, flux, operators); each group is one launch
+ * per LSRK stage and refinement level over a flat (domain, element) work
+ * list, the groups
  * run on forked streams, and a step is replayed from a CUDA graph.  The
  * domains keep their own state, time step and clock; a domain must not be
  * stepped by another stepper while it belongs to a batch.
@@ -437,8 +438,8 @@ int bfam_gpu_tile_shape(int dim, int N, int tile, int *threads,
                         int *min_ctas);
 /* elements per CTA of tile t (>= 1), or a negative BFAM_GPU_E* code */
 int bfam_gpu_tile_elements(int dim, int N, int tile);
-/* Choose group g's tile and persistent grid (ctas_per_sm CTAs per SM; 0:
- * as many as fit). */
+/* Choose group g's tile and the CTAs per SM its L2 lookahead assumes
+ * (ctas_per_sm; 0: as many as fit). */
 int bfam_gpu_batch_set_tile(bfam_gpu_batch_t *b, int g, int tile,
                             int ctas_per_sm);
 
