@@ -10,11 +10,11 @@
 // elements whatever the parity of Np, dq is loaded into registers ahead of the
 // barriers, and later items' rows are prefetched into L2, a line per thread.
 // Measured on 30 M DOF bricks, G DOF-updates/s before -> now (plain form,
-// conforming and with 30 % of the base cells refined): 2D N = 1 28 -> 85 and
-// 22 -> 63, N = 2 48 -> 112 and 36 -> 80, N = 3 82 -> 138 and 56 -> 113, N = 4
-// 81 -> 133 and 68 -> 107, N = 5 91 -> 138 and 65 -> 110, N = 6 81 -> 122 and
-// 67 -> 94, N = 7 141 -> 145 and 103 -> 118, N = 8 90 -> 115 and 79 -> 93; 3D
-// N = 1 56 -> 95 and 38 -> 62, N = 2 80 -> 97 and 58 -> 71.  Not used where the
+// conforming and with 30 % of the base cells refined): 2D N = 1 28 -> 86 and
+// 22 -> 63, N = 2 48 -> 117 and 36 -> 81, N = 3 82 -> 143 and 56 -> 116, N = 4
+// 81 -> 143 and 68 -> 110, N = 5 91 -> 143 and 65 -> 112, N = 6 81 -> 126 and
+// 67 -> 97, N = 7 141 -> 150 and 103 -> 118, N = 8 90 -> 118 and 79 -> 95; 3D
+// N = 1 56 -> 96 and 38 -> 62, N = 2 80 -> 98 and 58 -> 72.  Not used where the
 // one-element kernel is faster: 3D N = 3 (156 against 123) and 4, and the
 // precision form at 2D N = 7 (173 against 162).
 // What bounds it now is latency (long scoreboard) beside the LSU pipe (60 %).

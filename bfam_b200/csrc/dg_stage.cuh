@@ -105,10 +105,11 @@ __host__ __device__ constexpr int conforming_mode()
 // and after the node pass.  A thread per line between CTA barriers took 3,700
 // and 3,000 of the 20,800 cycles of an N = 7 element with two fine faces.
 // Refined meshes, G DOF-updates/s before -> with the projection -> with both:
-// N = 7 112.7 -> 118.4 -> 121.3, N = 6 112 -> 117 -> 118, N = 5 123 -> 130.1 ->
-// 130.4, N = 4 117 -> 118.5 -> 119.3, N = 3 115.9 -> 117.0 -> 117.9.  The plain
-// form's kernels here have no registers for it (N = 3 114 -> 110, N = 4 107 ->
-// 101).
+// N = 7 112.7 -> 118.4 -> 121.3, N = 6 112 -> 117 -> 118 (121 with the
+// differentiation rows of y and z from the parameter space), N = 5 123 -> 130.1
+// -> 130.4, N = 4 117 -> 118.5 -> 119.3 (122 with all rows from there), N = 3
+// 115.9 -> 117.0 -> 117.9.  The plain form's kernels here have no registers for
+// it (N = 3 114 -> 110, N = 4 107 -> 101).
 template <int DIM, int N, typename CT>
 __host__ __device__ constexpr bool mma_mortars()
 {

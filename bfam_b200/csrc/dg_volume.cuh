@@ -72,17 +72,29 @@ __device__ __forceinline__ CT line_ds(const CT *x, const CT *Dl)
 // data pipe is the busiest unit of the stage kernel; constant-cache reads
 // cost nothing there but serialise over the distinct rows of a warp.  A
 // warp's nodes share k at N = 5 (but for the last warp) and N = 7, and span
-// two k at N = 3.  Measured per shape (G DOF-updates/s against shared
-// rows): z alone +0.6 % (FP64) and +1 % (FP32) at N = 7, where all three
-// axes (eight distinct i) lost 3 and 9 %; all three axes +0.8 % at N = 3
-// (four distinct rows) in both forms and +0.6 % at N = 5 in FP64, where
-// FP32 lost 3.5 % with them and gains 0.4 % with z alone.  Other shapes
-// keep the shared copy.
+// two k at N = 3.  Measured per shape, 30 M DOFs, conforming meshes and
+// 30 % of the elements refined (rates against shared rows):
+//   3D N = 7: z alone +0.6 % (FP64), +1 % (FP32); all three axes (eight
+//     distinct i) -3 and -9 %.
+//   3D N = 6: y and z +2 % in FP32 (144.0 -> 147.5 G DOF-updates/s); FP64
+//     runs on the matrix instruction and reads no rows.
+//   3D N = 5: all three +0.6 % in FP64; in FP32 z alone +0.4 %, all -3.5 %.
+//   3D N <= 4 (at most five distinct rows): all three, +2.3 % at N = 4 in
+//     FP64 (140.2 -> 143.1, 108.7 -> 111.4) and +1 % in FP32, +0.8 % at
+//     N = 3 and 2, even at N = 1.
+//   2D N <= 4: both, +2.5 % at N = 2 (114.2 -> 117.0), +2.7 % at N = 3
+//     (139.2 -> 143.0), +5.5 % at N = 4 (135.2 -> 142.6) in FP64 and half
+//     of that in FP32, +0.5 % at N = 1.
+//   2D N = 6 and 8: y alone +2 % (123.1 -> 126.5, 115.5 -> 117.8) in both
+//     forms; x loses (FP32 N = 6 139 -> 129).  N = 5: y alone +1 % in FP32
+//     and -0.5 % on the refined mesh in FP64, which keeps the shared rows.
+//     N = 7: shared rows, y alone -3 % in FP64, both axes -18 %.
 template <int DIM, int N, typename CT> constexpr int dparam_axes()
 {
-  if (DIM != 3)
-    return 0;
-  return N == 3 ? 7 : N == 5 ? (sizeof(CT) == 8 ? 7 : 4) : N == 7 ? 4 : 0;
+  constexpr bool f64 = sizeof(CT) == 8;
+  if (DIM == 2)
+    return N <= 4 ? 3 : (N == 5 && !f64) || N == 6 || N == 8 ? 2 : 0;
+  return N <= 4 ? 7 : N == 5 ? (f64 ? 7 : 4) : N == 6 ? 6 : N == 7 ? 4 : 0;
 }
 
 // s times the volume right-hand side at node (i, j, k):
