@@ -121,6 +121,8 @@ struct TileImpl
 template <int DIM, int N, typename CT> struct PackTile
 {
   using K = PackShape<DIM, N, CT>;
+  using Small =
+      TileImpl<DIM, N, Shape<DIM, N>::NT, stage_min_ctas<DIM, N, CT>(), CT>;
   template <int MODE> static cudaError_t allow()
   {
     return cudaFuncSetAttribute(
@@ -132,16 +134,30 @@ template <int DIM, int N, typename CT> struct PackTile
                          const StageParams &sp, const double *hops, int,
                          cudaStream_t st, bool overlap)
   {
+    if constexpr (pack_has_small<DIM, N>())
+    {
+      constexpr int M =
+          MODE == MODE_STAGE_CF ? conforming_mode<DIM, N, CT>() : MODE;
+      if (pack_too_small<DIM, N>(nwork, sp.sms, MODE))
+        return Small::template run<M>(v, w, nwork, sp, hops, nwork, st,
+                                      overlap);
+    }
     const DiffOp<N, CT> dop = make_diffop<N, CT>(hops);
+    const StageParams pp = pack_params<DIM, N, K::E>(nwork, sp);
     return launch_dependent(overlap, dg_pack_batch_kernel<DIM, N, MODE, CT>,
-                            (nwork + K::E - 1) / K::E, K::NT, K::BYTES, st, v,
-                            w, nwork, sp, dop);
+                            pack_ctas(nwork, pp), K::NT, K::BYTES, st, v, w,
+                            nwork, pp, dop);
   }
   static cudaError_t prepare()
   {
     cudaError_t e = allow<MODE_STAGE>();
     if (e == cudaSuccess)
       e = allow<MODE_STAGE_NC>();
+    if constexpr (pack_has_small<DIM, N>())
+    {
+      if (e == cudaSuccess)
+        e = Small::prepare();
+    }
     return e == cudaSuccess ? allow<MODE_STAGE_CF>() : e;
   }
   static int occupancy()
@@ -675,6 +691,7 @@ int issue_step(bfam_gpu_batch_t *b, int p)
       sp.first_stage = s == 0;
       sp.flux = g.flux;
       sp.ahead = g.ahead;
+      sp.sms = b->sms;
       // levels in order: coarse elements after the fine ones across their
       // hanging faces
       for (size_t l = 0; l < g.work.size(); ++l)
@@ -765,6 +782,7 @@ int issue_step_glued(bfam_gpu_batch_t *b, int p)
       sp.first_stage = s == 0;
       sp.flux = g.flux;
       sp.ahead = g.ahead;
+      sp.sms = b->sms;
       for (size_t l = 0; l < g.work.size(); ++l)
       {
         if (int rc = launch_level(b, g, l, par, sp, st, false))

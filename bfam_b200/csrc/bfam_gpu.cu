@@ -73,6 +73,24 @@ cudaError_t mma_launch(const DomainView &v, int n, const StageParams &sp,
                           1.0 / hops[7 * (N + 1) * (N + 1)]);
 }
 
+// a thread per node, a CTA per element
+template <int DIM, int N, typename CT>
+cudaError_t node_launch(const DomainView &v, int n, const StageParams &sp,
+                        const double *hops, int mode, cudaStream_t stream,
+                        bool overlap)
+{
+  using S = Shape<DIM, N>;
+  const DiffOp<N, CT> dop = make_diffop<N, CT>(hops);
+  const size_t smem = stage_smem_bytes<DIM, N, CT>();
+  return launch_dependent(
+      overlap,
+      mode == MODE_STAGE      ? single_kernel<DIM, N, CT, MODE_STAGE>
+      : mode == MODE_STAGE_NC ? single_kernel<DIM, N, CT, MODE_STAGE_NC>
+      : mode == MODE_STAGE_CF ? single_kernel<DIM, N, CT, conforming_mode<DIM, N, CT>()>
+                              : single_kernel<DIM, N, CT, MODE_RHS>,
+      n, S::NT, smem, stream, v, n, sp, dop);
+}
+
 // n work items, a CTA for each element (packed: for several)
 template <int DIM, int N, typename CT>
 cudaError_t stage_launch(const DomainView &v, int n, const StageParams &sp,
@@ -84,33 +102,28 @@ cudaError_t stage_launch(const DomainView &v, int n, const StageParams &sp,
     if (mma_for_mesh<N>(hops))
       return mma_launch<N>(v, n, sp, hops, mode, stream, overlap);
   }
+  if constexpr (pack_has_small<DIM, N>())
+  {
+    if (pack_too_small<DIM, N>(n, sp.sms, mode))
+      return node_launch<DIM, N, CT>(v, n, sp, hops, mode, stream, overlap);
+  }
   if constexpr (use_mma<DIM, N, CT>())
     return mma_launch<N>(v, n, sp, hops, mode, stream, overlap);
   else if constexpr (use_pack<DIM, N, CT>())
   {
     using K = PackShape<DIM, N, CT>;
     const DiffOp<N, CT> dop = make_diffop<N, CT>(hops);
+    const StageParams pp = pack_params<DIM, N, K::E>(n, sp);
     return launch_dependent(
         overlap,
         mode == MODE_STAGE      ? dg_pack_kernel<DIM, N, MODE_STAGE, CT>
         : mode == MODE_STAGE_NC ? dg_pack_kernel<DIM, N, MODE_STAGE_NC, CT>
         : mode == MODE_STAGE_CF ? dg_pack_kernel<DIM, N, MODE_STAGE_CF, CT>
                                 : dg_pack_kernel<DIM, N, MODE_RHS, CT>,
-        (n + K::E - 1) / K::E, K::NT, K::BYTES, stream, v, n, sp, dop);
+        pack_ctas(n, pp), K::NT, K::BYTES, stream, v, n, pp, dop);
   }
   else
-  {
-    using S = Shape<DIM, N>;
-    const DiffOp<N, CT> dop = make_diffop<N, CT>(hops);
-    const size_t smem = stage_smem_bytes<DIM, N, CT>();
-    return launch_dependent(
-        overlap,
-        mode == MODE_STAGE      ? single_kernel<DIM, N, CT, MODE_STAGE>
-        : mode == MODE_STAGE_NC ? single_kernel<DIM, N, CT, MODE_STAGE_NC>
-        : mode == MODE_STAGE_CF ? single_kernel<DIM, N, CT, conforming_mode<DIM, N, CT>()>
-                                : single_kernel<DIM, N, CT, MODE_RHS>,
-        n, S::NT, smem, stream, v, n, sp, dop);
-  }
+    return node_launch<DIM, N, CT>(v, n, sp, hops, mode, stream, overlap);
 }
 
 template <typename K> cudaError_t allow_smem(K kernel, int bytes)
@@ -154,6 +167,19 @@ template <int DIM, int N, typename CT> cudaError_t stage_prepare(int *occ)
     if (e == cudaSuccess)
       e = occupancy(dg_pack_kernel<DIM, N, MODE_RHS, CT>, K::NT, K::BYTES,
                     &occ[MODE_RHS]);
+    if constexpr (pack_has_small<DIM, N>())
+    {
+      const int smem = (int)stage_smem_bytes<DIM, N, CT>();
+      if (e == cudaSuccess)
+        e = allow_smem(single_kernel<DIM, N, CT, MODE_STAGE>, smem);
+      if (e == cudaSuccess)
+        e = allow_smem(single_kernel<DIM, N, CT, MODE_STAGE_NC>, smem);
+      if (e == cudaSuccess)
+        e = allow_smem(
+            single_kernel<DIM, N, CT, conforming_mode<DIM, N, CT>()>, smem);
+      if (e == cudaSuccess)
+        e = allow_smem(single_kernel<DIM, N, CT, MODE_RHS>, smem);
+    }
     return e;
   }
   else
@@ -436,6 +462,7 @@ int launch_stage(bfam_gpu_domain_t *d, int in, double A, double B, double C,
   // prefetch part of a wave of resident CTAs ahead (half a wave: about half a
   // CTA lifetime before the element's CTA starts)
   sp.ahead = d->ks.occ[mode] * d->sms * d->ks.elements / d->ks.lookahead;
+  sp.sms = d->sms;
   DomainView v = view(d, in);
   v.dt = dt;
   // one launch per level; level l's elements after level l-1's

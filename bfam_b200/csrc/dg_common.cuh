@@ -83,6 +83,8 @@ struct StageParams
   // element of item i + ahead (half a wave of resident CTAs later), so that
   // its loads find L2 (0: no prefetch)
   int ahead;
+  int sms;     // SMs of the device
+  int per = 0; // packed kernel: elements per CTA, set by its launch
 };
 
 // Ricker wavelet (1 - 2 a) exp(-a), a = (pi f0 (t - t0))^2

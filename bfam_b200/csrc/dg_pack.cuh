@@ -65,6 +65,51 @@ __host__ __device__ constexpr bool use_pack()
   return DIM == 2 ? N != 7 || sizeof(CT) == sizeof(double) : N <= 2;
 }
 
+// Low orders, whose CTA holds many elements: on a small mesh a CTA takes only
+// so many that every SM gets four CTAs.  The passes before the node pass run
+// over a CTA's faces, so fewer elements per CTA shorten the chain of latencies
+// that bounds a small mesh (us per step, full CTAs -> spread; one element per
+// CTA of the node-per-thread kernel in brackets): 2D N = 1, 1,822 refined
+// elements 47 -> 36 (38), 6,895 50 -> 38 (58); 2D N = 2, 1,822 46 -> 37 (42);
+// 3D N = 1, 398 67 -> 40 (53), 6,425 85 -> 66 (96); 3D N = 2, 398 67 -> 53
+// (52).  One CTA per SM instead of four: 36, 45, 38, 40, 79, 62.  At the other
+// orders (two to eight elements per CTA) it gave nothing and the variable
+// count cost 2-6 % (2D N = 6 397 -> 415), so it is a constant there.
+template <int DIM, int N> __host__ __device__ constexpr bool pack_spreads()
+{
+  return N <= 2;
+}
+
+// sp with the elements per CTA for n elements
+template <int DIM, int N, int E>
+inline StageParams pack_params(int n, StageParams sp)
+{
+  const int spread = (n + 4 * sp.sms - 1) / (4 * sp.sms);
+  sp.per = pack_spreads<DIM, N>() && spread < E ? spread : E;
+  return sp;
+}
+
+inline int pack_ctas(int n, const StageParams &sp)
+{
+  return (n + sp.per - 1) / sp.per;
+}
+
+// Launches of a served shape that are too small for it: at 3D N = 2 a CTA's
+// four elements have up to 12 fine faces and its 128 threads go through their
+// lines in turns, so below 48 elements per SM the node-per-thread kernel's many
+// small CTAs are faster (us per step packed and not: 398 refined elements 53
+// and 48, 1,597 76 and 60, 6,425 157 and 145, the few coarse-sided elements of
+// 28,168 553 and 533); without hanging faces below 12 (512 elements 25.4 and
+// 23.4, 1,728 42 and 35 in the precision form, 4,096 69 and 71).
+template <int DIM, int N> constexpr bool pack_has_small()
+{
+  return DIM == 3 && N == 2;
+}
+template <int DIM, int N> bool pack_too_small(int n, int sms, int mode)
+{
+  return pack_has_small<DIM, N>() && n < (mode == MODE_STAGE_CF ? 12 : 48) * sms;
+}
+
 // The 1-D mortar pass of line_apply on `lines` faces of NC fields each (2D
 // orders 6 and up), a thread per value instead of per line: a CTA has few
 // lines there, and a thread per line left most of it waiting for Nq x Nq
@@ -134,8 +179,9 @@ __device__ __forceinline__ void pack_elements(const Item &item, int n,
   int *fidx = reinterpret_cast<int *>(desc + K::E * NF); // mortar slot or -1
   int *elem = fidx + K::E * NF;
   int *flist = elem + K::E, *fcount = flist + K::E * DIM;
-  const int t = threadIdx.x, first = blockIdx.x * K::E;
-  const int ne = n - first < K::E ? n - first : K::E; // elements here
+  const int t = threadIdx.x, per = pack_spreads<DIM, N>() ? sp.per : K::E;
+  const int first = blockIdx.x * per;
+  const int ne = n - first < per ? n - first : per; // elements here
   const bool rd = MODE != MODE_RHS && !sp.first_stage;
   constexpr bool HANGS = MODE != MODE_STAGE_CF; // any hanging face
 
@@ -220,7 +266,7 @@ __device__ __forceinline__ void pack_elements(const Item &item, int n,
   if (sp.ahead > 0)
   {
     constexpr int L = (Np * 8 + 127) / 128 + (Np % 16 ? 1 : 0);
-    for (int w = t; w < K::E * L; w += NT)
+    for (int w = t; w < per * L; w += NT)
     {
       const int ia = first + sp.ahead + w / L;
       if (ia < n)
@@ -449,7 +495,7 @@ __device__ __forceinline__ void pack_elements(const Item &item, int n,
   }
 }
 
-// one domain: CTA b takes work items b E, b E + 1, ...
+// one domain: CTA b takes the work items from b sp.per on
 template <int DIM, int N, int MODE, typename CT>
 __global__ void __launch_bounds__(PackShape<DIM, N, CT>::NT,
                                   PackShape<DIM, N, CT>::MINB)

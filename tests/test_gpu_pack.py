@@ -71,3 +71,34 @@ def test_domains_meeting_inside_a_cta(dim, N, prec):
         assert np.array_equal(d.get_fields(), q)
         assert np.array_equal(d.seismograms(), s)
     b.free()
+
+
+# Meshes whose launches give a CTA two, several or all of the elements that it
+# can hold, with a partly empty last CTA, and (3D order 2) launches on either
+# side of the size from which the packed kernel serves them.  The counts are of
+# the finest level's order: 4 x 148 CTAs before a second element per CTA.
+SPREAD = [(2, 1, (29, 23), 0.0), (2, 1, (51, 37), 0.4), (2, 1, (140, 137), 0.0),
+          (2, 2, (27, 23), 0.0), (2, 2, (43, 31), 0.4), (2, 2, (97, 89), 0.3),
+          (3, 1, (9, 10, 7), 0.0), (3, 1, (9, 8, 7), 0.4), (3, 1, (23, 21, 20), 0.2),
+          (3, 2, (11, 12, 13), 0.0), (3, 2, (13, 12, 12), 0.0), (3, 2, (8, 7, 7), 0.4),
+          (3, 2, (16, 14, 15), 0.3)]
+
+
+@pytest.mark.parametrize("dim,N,n,p", SPREAD, ids=str)
+@pytest.mark.parametrize("prec,tol", [(bf.PRECISION_FP64, 1e-12), (bf.PRECISION_FP32, 1e-6)],
+                         ids=["fp64", "fp32"])
+def test_elements_per_cta(dim, N, n, p, prec, tol):
+    m, rho, lam, mu, q, dt = _problem(dim, N, n, p, N, False)
+    o = orc.Oracle.from_mesh(m, rho, lam, mu, 0)
+    ref = o.lsrk(q, dt, 1)
+    doms = []
+    for _ in range(3):
+        d = bf.GpuDomain(m, rho, lam, mu, precision=prec)
+        d.set_fields(q)
+        doms.append(d)
+    bf.LSRK(doms[0]).step(dt, 1)
+    alone = doms[0].get_fields()
+    assert relerr(alone, ref).max() < tol
+    bf.Batch(doms[1:]).step([dt, dt], 1)
+    for d in doms[1:]:
+        assert np.array_equal(d.get_fields(), alone)
