@@ -322,7 +322,7 @@ def run_reference(args):
 
 
 def run_batched(args):
-    """cfg3: many independent instances in one batch (one persistent launch
+    """cfg3: many independent instances in one batch (one launch
     per order group and stage, graph-replayed steps, autotuned tiles)."""
     import torch
     ws, rank, local = dist_init()
@@ -857,11 +857,12 @@ def main():
     alg_bytes_per_stage = p.ndof * ALG_BYTES_PER_DOF_UPDATE[ns]
     achieved = alg_bytes_per_stage / per_stage_s / 1e9
     peak, peak_kind = measured_peak()
-    traffic = profiled_traffic(f"dg_stage_kernel_{p.name}") if p.mesh.dim == 3 else None
+    traffic = profiled_traffic(f"stage_{p.name}") if p.mesh.dim == 3 else None
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "peak_source": f"of {peak_kind}",
                 "traffic": traffic,
-                "kernel": "dg_stage_kernel (fused volume+face+mortar+LSRK update)",
+                "kernel": ("dg_stage_kernel" if prec == bf.PRECISION_FP32 else "dg_mma_kernel") +
+                " (fused volume+face+mortar+LSRK update)",
                 "per": f"LSRK stage = {levels} launch(es), one per refinement level",
                 "alg_bytes_per_stage": alg_bytes_per_stage,
                 "launches_per_stage": levels}
