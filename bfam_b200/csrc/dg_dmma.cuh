@@ -75,8 +75,8 @@ __device__ __forceinline__ void mortar_pair(const double *ops, int op, int hp,
 {
   constexpr int Nq = N + 1, P = Nq * Nq;
   const int rr = (threadIdx.x & 31) >> 2, c = threadIdx.x & 3;
-  // lanes past the matrix repeat its last row and column: finite values
-  // that meet zeros of the operator or are not stored
+  // lanes past the matrix read its last row and column; their values are not
+  // stored, and zeros where they meet the operator's
   const int r = rr < Nq ? rr : N;
   const int i0 = 2 * c < Nq ? 2 * c : N, i1 = 2 * c + 1 < Nq ? 2 * c + 1 : N;
   auto frag = [&](int top) {
@@ -91,6 +91,13 @@ __device__ __forceinline__ void mortar_pair(const double *ops, int op, int hp,
                       x0[fpos<3, N>(g0, i1 + Nq * r)]);
   y[1] = make_double2(x1[fpos<3, N>(g1, i0 + Nq * r)],
                       x1[fpos<3, N>(g1, i1 + Nq * r)]);
+  if (Nq < 8)
+  {
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+      y[k] = make_double2(rr < Nq && 2 * c < Nq ? y[k].x : 0.0,
+                          rr < Nq && 2 * c + 1 < Nq ? y[k].y : 0.0);
+  }
   dmma_t<2>(a, y);
   dmma_t<2>(b, y);
 }

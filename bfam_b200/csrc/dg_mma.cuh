@@ -153,8 +153,8 @@ __device__ __forceinline__ void mma_element(const Item &item, int n,
   uint64_t *bar = reinterpret_cast<uint64_t *>(smem + M::OFF_BAR);
   const int t = threadIdx.x, w = t >> 5, rr = (t & 31) >> 2, c = t & 3;
   // row and columns of this lane; lanes past the matrix read its last row
-  // or columns instead (their products meet zero operator entries or land
-  // in rows and columns that are not stored)
+  // or columns instead (they land in rows and columns that are not stored;
+  // as entries past a contracted index they are replaced by zeros)
   const bool v0 = rr < Nq && 2 * c < Nq, v1 = rr < Nq && 2 * c + 1 < Nq;
   const int r = rr < Nq ? rr : N;
   const int i0 = 2 * c < Nq ? 2 * c : (VEC ? N - 1 : N);
@@ -320,7 +320,7 @@ __device__ __forceinline__ void mma_element(const Item &item, int n,
       for (int q = 0; q < 6; ++q)
       {
         const int f = q == 0 ? 7 : q == 1 ? 8 : q == 2 ? 5 : q - 3;
-        dmma(z[q], fz.y, row(f)[w * Nq + o1z]);
+        dmma(z[q], fz.y, k1 < Nq ? row(f)[w * Nq + o1z] : 0.0);
       }
       double *o = zrow(0, r, w) + i0;
       if (v0)
@@ -351,6 +351,12 @@ __device__ __forceinline__ void mma_element(const Item &item, int n,
     // operators, three at a time; the result has columns 2 c and 2 c + 1
     auto tensor = [&](int op) {
       const bool y4 = N == 7 && da == 4;
+      if (Nq < 8)
+      {
+#pragma unroll
+        for (int q = 0; q < 6; ++q)
+          nb[q] = make_double2(v0 ? nb[q].x : 0.0, v1 ? nb[q].y : 0.0);
+      }
       const double2 oa = frag(op, (hp - 1) & 1, y4 ? c : 2 * c, y4 ? c + 4 : 2 * c + 1),
                     ob = frag(op, (hp - 1) >> 1, 2 * c, 2 * c + 1);
 #pragma unroll
@@ -466,6 +472,8 @@ __device__ __forceinline__ void mma_element(const Item &item, int n,
   const int y0 = YS ? c : 2 * c, y1 = YS ? c + 4 : 2 * c + 1;
   const int oy0 = w * PP + (y0 < Nq ? y0 : N) * Nq + r,
             oy1 = w * PP + (y1 < Nq ? y1 : N) * Nq + r;
+  // y0 and y1 are indices of a row, for the lanes whose results are stored
+  const bool yk0 = N != 5 || v0, yk1 = N == 7 || v1;
   auto startx = [&](int q) {
     double2 y = make_double2(0.0, 0.0);
     if (xl)
@@ -484,14 +492,18 @@ __device__ __forceinline__ void mma_element(const Item &item, int n,
   };
   auto dxy = [&](int f, int jx, int g, int jy, double2 &X, double2 &Y) {
     double2 x = make_double2(0.0, 0.0);
-    if (rr < Nq)
-      x = get2<VEC>(row(f) + m0, o1);
+    if (VEC && v0)
+      x = get2<true>(row(f) + m0);
+    if (!VEC && v0)
+      x.x = row(f)[m0];
+    if (!VEC && v1)
+      x.y = row(f)[m0 + 1];
     X = startx(jx);
     Y = starty(jy);
     dmma(X, x.x, fx.x);
-    dmma(Y, fy.x, row(g)[oy0]);
+    dmma(Y, fy.x, yk0 ? row(g)[oy0] : 0.0);
     dmma(X, x.y, fx.y);
-    dmma(Y, fy.y, row(g)[oy1]);
+    dmma(Y, fy.y, yk1 ? row(g)[oy1] : 0.0);
   };
   // the derivative along z with its faces' corrections (jump component jq)
   const double *pz = zrow(0, w, r) + i0;
