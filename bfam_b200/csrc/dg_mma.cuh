@@ -306,6 +306,7 @@ __device__ __forceinline__ void mma_element(const Item &item, int n,
     const int o0 = (k0 < Nq ? k0 : N) * PP + r, o1z = (k1 < Nq ? k1 : N) * PP + r;
     if (!mbar_wait(bar, 0))
       atomicExch(d.err, 1);
+    __syncwarp(); // the matrix instruction takes whole warps
     {
       double2 z[6];
 #pragma unroll

@@ -715,6 +715,7 @@ __device__ __forceinline__ void compute_element(const DomainView &d,
   // second pass of nodes): no other warp waits for it
   if constexpr (HANGS && MMA)
   {
+    __syncwarp(); // the matrix instruction takes whole warps
     for (int w = NW - 1 - wid; w < 3 * nfine; w += NW)
     {
       const int fr = w / 3, c = w % 3, f = nth_bit(fine_mask, fr);
