@@ -181,6 +181,7 @@ def _declare(L: C.CDLL) -> None:
                                           P(C.c_int)]),
         "bfam_gpu_batch_set_tile": (C.c_int, [vp, C.c_int, C.c_int, C.c_int]),
         "bfam_gpu_launch_count": (C.c_uint64, []),
+        "bfam_gpu_prepare_count": (C.c_uint64, []),
         "bfam_gpu_last_error": (C.c_int, [C.c_char_p, C.c_size_t]),
         "bfam_gpu_record_error": (C.c_int, [C.c_int, C.c_char_p]),
         "bfam_gpu_trim_pool": (C.c_int, [C.c_int, C.c_size_t]),
@@ -215,6 +216,11 @@ def _ptrs(arrs) -> C.Array:
 
 def launch_count() -> int:
     return int(lib().bfam_gpu_launch_count())
+
+
+def prepare_count() -> int:
+    """stage kernels set up for launching since process start"""
+    return int(lib().bfam_gpu_prepare_count())
 
 
 # ----------------------------------------------------------------- operators

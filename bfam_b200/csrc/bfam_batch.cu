@@ -35,8 +35,9 @@ namespace
 typedef cudaError_t (*batch_launch_fn)(const DomainView *, const int2 *, int,
                                 const StageParams &, const double *hops,
                                 int grid, cudaStream_t, bool overlap);
-typedef cudaError_t (*batch_prepare_fn)();
-typedef int (*batch_occupancy_fn)();
+// for launches of n elements in one stage mode
+typedef cudaError_t (*batch_prepare_fn)(int mode, int n, int sms);
+typedef int (*batch_occupancy_fn)(int mode);
 
 struct BatchTile
 {
@@ -61,6 +62,27 @@ struct BatchTile
   batch_occupancy_fn occupancy = nullptr;
 };
 
+// shared-memory opt-in, and resident CTAs per SM (0: none), of a tile's kernel
+template <typename K> cudaError_t allow_smem(K kernel, size_t smem)
+{
+  g_prepares.fetch_add(1, std::memory_order_relaxed);
+  return cudaFuncSetAttribute((const void *)kernel,
+                              cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)smem);
+}
+
+template <typename K> int resident(K kernel, int threads, size_t smem)
+{
+  int n = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem) !=
+      cudaSuccess)
+  {
+    cudaGetLastError();
+    return 0;
+  }
+  return n;
+}
+
 template <int DIM, int N, int NT, int MINB, typename CT, int EPC = 1>
 struct TileImpl
 {
@@ -77,30 +99,17 @@ struct TileImpl
     return launch_dependent(overlap, kernel<MODE>, grid, NT * EPC, SMEM, st, v,
                             w, nwork, sp, dop);
   }
-  template <int MODE> static cudaError_t allow()
+  static auto of(int mode)
   {
-    return cudaFuncSetAttribute((const void *)kernel<MODE>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)SMEM);
+    return mode == MODE_STAGE_CF   ? kernel<conforming_mode<DIM, N, CT>()>
+           : mode == MODE_STAGE_NC ? kernel<MODE_STAGE_NC>
+                                   : kernel<MODE_STAGE>;
   }
-  static cudaError_t prepare()
+  static cudaError_t prepare(int mode, int, int)
   {
-    cudaError_t e = allow<MODE_STAGE>();
-    if (e == cudaSuccess)
-      e = allow<MODE_STAGE_NC>();
-    return e == cudaSuccess ? allow<conforming_mode<DIM, N, CT>()>() : e;
+    return allow_smem(of(mode), SMEM);
   }
-  static int occupancy()
-  {
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &n, kernel<MODE_STAGE>, NT * EPC, SMEM) != cudaSuccess)
-    {
-      cudaGetLastError();
-      return 0;
-    }
-    return n;
-  }
+  static int occupancy(int mode) { return resident(of(mode), NT * EPC, SMEM); }
   static BatchTile make()
   {
     BatchTile t;
@@ -123,12 +132,6 @@ template <int DIM, int N, typename CT> struct PackTile
   using K = PackShape<DIM, N, CT>;
   using Small =
       TileImpl<DIM, N, Shape<DIM, N>::NT, stage_min_ctas<DIM, N, CT>(), CT>;
-  template <int MODE> static cudaError_t allow()
-  {
-    return cudaFuncSetAttribute(
-        (const void *)dg_pack_batch_kernel<DIM, N, MODE, CT>,
-        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)K::BYTES);
-  }
   template <int MODE>
   static cudaError_t run(const DomainView *v, const int2 *w, int nwork,
                          const StageParams &sp, const double *hops, int,
@@ -148,30 +151,22 @@ template <int DIM, int N, typename CT> struct PackTile
                             pack_ctas(nwork, pp), K::NT, K::BYTES, st, v, w,
                             nwork, pp, dop);
   }
-  static cudaError_t prepare()
+  static auto of(int mode)
   {
-    cudaError_t e = allow<MODE_STAGE>();
-    if (e == cudaSuccess)
-      e = allow<MODE_STAGE_NC>();
+    return mode == MODE_STAGE_CF   ? dg_pack_batch_kernel<DIM, N, MODE_STAGE_CF, CT>
+           : mode == MODE_STAGE_NC ? dg_pack_batch_kernel<DIM, N, MODE_STAGE_NC, CT>
+                                   : dg_pack_batch_kernel<DIM, N, MODE_STAGE, CT>;
+  }
+  static cudaError_t prepare(int mode, int n, int sms)
+  {
     if constexpr (pack_has_small<DIM, N>())
     {
-      if (e == cudaSuccess)
-        e = Small::prepare();
+      if (pack_too_small<DIM, N>(n, sms, mode))
+        return Small::prepare(mode, n, sms);
     }
-    return e == cudaSuccess ? allow<MODE_STAGE_CF>() : e;
+    return allow_smem(of(mode), K::BYTES);
   }
-  static int occupancy()
-  {
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &n, dg_pack_batch_kernel<DIM, N, MODE_STAGE, CT>, K::NT, K::BYTES) !=
-        cudaSuccess)
-    {
-      cudaGetLastError();
-      return 0;
-    }
-    return n;
-  }
+  static int occupancy(int mode) { return resident(of(mode), K::NT, K::BYTES); }
   static BatchTile make()
   {
     BatchTile t;
@@ -210,23 +205,11 @@ template <int N, int MINB> struct MmaTile
     return launch_dependent(overlap, kernel, grid, M::NT, M::BYTES, st, v, w, nwork, sp,
                             1.0 / hops[7 * (N + 1) * (N + 1)]);
   }
-  static cudaError_t prepare()
+  static cudaError_t prepare(int, int, int)
   {
-    return cudaFuncSetAttribute((const void *)kernel,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)M::BYTES);
+    return allow_smem(kernel, M::BYTES);
   }
-  static int occupancy()
-  {
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, M::NT,
-                                                      M::BYTES) != cudaSuccess)
-    {
-      cudaGetLastError();
-      return 0;
-    }
-    return n;
-  }
+  static int occupancy(int) { return resident(kernel, M::NT, M::BYTES); }
   static BatchTile make()
   {
     BatchTile t;
@@ -565,11 +548,32 @@ void drop_graphs(bfam_gpu_batch_t *b)
     }
 }
 
+// stage mode of the group's l-th launch
+int group_mode(const bfam_gpu_batch::Group &g, size_t l)
+{
+  return l > 0 || !g.level0_nc ? MODE_STAGE
+         : g.conforming        ? MODE_STAGE_CF
+                               : MODE_STAGE_NC;
+}
+
+// A group of one domain under the default tile runs the single-domain kernel
+// (the same arithmetic with the domain's view in the parameter bank: at N = 5
+// in FP64 the batch kernel, which reads its view from memory, spills at five
+// CTAs per SM).
+bool alone(const bfam_gpu_batch::Group &g)
+{
+  return g.doms.size() == 1 && g.tile == 0 && g.ctas_per_sm == 0;
+}
+
 int choose_grid(bfam_gpu_batch_t *b, bfam_gpu_batch_t::Group &g)
 {
+  if (alone(g)) // the single-domain kernel, set up with its domain
+    return 0;
   const BatchTile &t = g.tiles[g.tile];
-  CUDA_TRY(t.prepare());
-  int occ = t.occupancy();
+  // the kernels that the group's levels launch
+  for (size_t l = 0; l < g.work.size(); ++l)
+    CUDA_TRY(t.prepare(group_mode(g, l), (int)g.nwork_l[l], b->sms));
+  int occ = t.occupancy(group_mode(g, 0));
   if (occ <= 0)
     return fail(BFAM_GPU_EUNSUPPORTED,
                 "tile %d (%d threads) of order %d does not fit on an SM",
@@ -637,17 +641,12 @@ cudaError_t launch_post_step(bfam_gpu_batch_t *b, int p)
                           POST_THREADS, 0, b->stream, b->post[p]);
 }
 
-// Level l of group g's stage sp, from state parity par.  A group of one domain
-// under the default tile runs the single-domain kernel (the same arithmetic
-// with the domain's view in the parameter bank: at N = 5 in FP64 the batch
-// kernel, which reads its view from memory, spills at five CTAs per SM).
+// Level l of group g's stage sp, from state parity par.
 int launch_level(bfam_gpu_batch_t *b, bfam_gpu_batch::Group &g, size_t l,
                  int par, const StageParams &sp, cudaStream_t st, bool overlap)
 {
-  const int mode = l > 0 || !g.level0_nc ? MODE_STAGE
-                   : g.conforming         ? MODE_STAGE_CF
-                                          : MODE_STAGE_NC;
-  if (g.doms.size() == 1 && g.tile == 0 && g.ctas_per_sm == 0)
+  const int mode = group_mode(g, l);
+  if (alone(g))
   {
     const int i = g.doms[0];
     bfam_gpu_domain_t *d = b->doms[i];
@@ -655,9 +654,7 @@ int launch_level(bfam_gpu_batch_t *b, bfam_gpu_batch::Group &g, size_t l,
     v.dt = b->dt[i];
     if (d->nlevels > 1)
       v.elist = d->elist + d->level_off[l];
-    CUDA_TRY(d->ks.launch(v, (int)g.nwork_l[l], sp, g.hops.data(),
-                          mode, st, overlap));
-    return 0;
+    return launch_elements(d, v, (int)g.nwork_l[l], sp, mode, st, overlap);
   }
   const BatchTile &t = g.tiles[g.tile];
   CUDA_TRY(t.of(mode)(g.views[par], g.work[l], (int)g.nwork_l[l], sp,

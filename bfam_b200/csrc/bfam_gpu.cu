@@ -34,6 +34,7 @@ namespace host
 
 thread_local std::string g_err;
 std::atomic<uint64_t> g_launches{0};
+std::atomic<uint64_t> g_prepares{0};
 
 int fail(int code, const char *fmt, ...)
 {
@@ -91,122 +92,119 @@ cudaError_t node_launch(const DomainView &v, int n, const StageParams &sp,
       n, S::NT, smem, stream, v, n, sp, dop);
 }
 
+// The kernel of a launch over n elements.
+template <int DIM, int N, typename CT>
+int stage_kernel(int n, const double *hops, int sms, int mode)
+{
+  if constexpr (use_mma_hanging<DIM, N, CT>())
+  {
+    if (mma_for_mesh<N>(hops))
+      return KERNEL_MMA;
+  }
+  if constexpr (pack_has_small<DIM, N>())
+  {
+    if (pack_too_small<DIM, N>(n, sms, mode))
+      return KERNEL_NODE;
+  }
+  return use_mma<DIM, N, CT>()    ? KERNEL_MMA
+         : use_pack<DIM, N, CT>() ? KERNEL_PACK
+                                  : KERNEL_NODE;
+}
+
+// several elements per CTA
+template <int DIM, int N, typename CT, int MODE>
+constexpr auto pack_kernel = dg_pack_kernel<DIM, N, MODE, CT>;
+
+template <int DIM, int N, typename CT>
+cudaError_t pack_launch(const DomainView &v, int n, const StageParams &sp,
+                        const double *hops, int mode, cudaStream_t stream,
+                        bool overlap)
+{
+  using K = PackShape<DIM, N, CT>;
+  const DiffOp<N, CT> dop = make_diffop<N, CT>(hops);
+  const StageParams pp = pack_params<DIM, N, K::E>(n, sp);
+  return launch_dependent(
+      overlap,
+      mode == MODE_STAGE      ? pack_kernel<DIM, N, CT, MODE_STAGE>
+      : mode == MODE_STAGE_NC ? pack_kernel<DIM, N, CT, MODE_STAGE_NC>
+      : mode == MODE_STAGE_CF ? pack_kernel<DIM, N, CT, MODE_STAGE_CF>
+                              : pack_kernel<DIM, N, CT, MODE_RHS>,
+      pack_ctas(n, pp), K::NT, K::BYTES, stream, v, n, pp, dop);
+}
+
 // n work items, a CTA for each element (packed: for several)
 template <int DIM, int N, typename CT>
 cudaError_t stage_launch(const DomainView &v, int n, const StageParams &sp,
                          const double *hops, int mode, cudaStream_t stream,
                          bool overlap)
 {
-  if constexpr (use_mma_hanging<DIM, N, CT>())
+  const int k = stage_kernel<DIM, N, CT>(n, hops, sp.sms, mode);
+  if constexpr (use_mma<DIM, N, CT>() || use_mma_hanging<DIM, N, CT>())
   {
-    if (mma_for_mesh<N>(hops))
+    if (k == KERNEL_MMA)
       return mma_launch<N>(v, n, sp, hops, mode, stream, overlap);
   }
-  if constexpr (pack_has_small<DIM, N>())
+  if constexpr (use_pack<DIM, N, CT>())
   {
-    if (pack_too_small<DIM, N>(n, sp.sms, mode))
-      return node_launch<DIM, N, CT>(v, n, sp, hops, mode, stream, overlap);
+    if (k == KERNEL_PACK)
+      return pack_launch<DIM, N, CT>(v, n, sp, hops, mode, stream, overlap);
   }
-  if constexpr (use_mma<DIM, N, CT>())
-    return mma_launch<N>(v, n, sp, hops, mode, stream, overlap);
-  else if constexpr (use_pack<DIM, N, CT>())
-  {
-    using K = PackShape<DIM, N, CT>;
-    const DiffOp<N, CT> dop = make_diffop<N, CT>(hops);
-    const StageParams pp = pack_params<DIM, N, K::E>(n, sp);
-    return launch_dependent(
-        overlap,
-        mode == MODE_STAGE      ? dg_pack_kernel<DIM, N, MODE_STAGE, CT>
-        : mode == MODE_STAGE_NC ? dg_pack_kernel<DIM, N, MODE_STAGE_NC, CT>
-        : mode == MODE_STAGE_CF ? dg_pack_kernel<DIM, N, MODE_STAGE_CF, CT>
-                                : dg_pack_kernel<DIM, N, MODE_RHS, CT>,
-        pack_ctas(n, pp), K::NT, K::BYTES, stream, v, n, pp, dop);
-  }
-  else
+  if constexpr (!use_mma<DIM, N, CT>() &&
+                (!use_pack<DIM, N, CT>() || pack_has_small<DIM, N>()))
     return node_launch<DIM, N, CT>(v, n, sp, hops, mode, stream, overlap);
+  else
+    return cudaErrorInvalidDeviceFunction;
 }
 
-template <typename K> cudaError_t allow_smem(K kernel, int bytes)
-{
-  return cudaFuncSetAttribute((const void *)kernel,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              bytes);
-}
-
+// shared-memory opt-in of one kernel, and its resident CTAs per SM
 template <typename K>
-cudaError_t occupancy(K kernel, int threads, size_t smem, int *occ)
+cudaError_t prepare_one(K kernel, int threads, size_t smem, int *occ)
 {
-  const cudaError_t e = allow_smem(kernel, (int)smem);
+  g_prepares.fetch_add(1, std::memory_order_relaxed);
+  const cudaError_t e =
+      smem <= 48 * 1024
+          ? cudaSuccess
+          : cudaFuncSetAttribute((const void *)kernel,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)smem);
   return e != cudaSuccess ? e
                           : cudaOccupancyMaxActiveBlocksPerMultiprocessor(
                                 occ, kernel, threads, smem);
 }
 
-// shared-memory opt-in, and the resident CTAs per SM of both modes
-template <int DIM, int N, typename CT> cudaError_t stage_prepare(int *occ)
+template <int DIM, int N, typename CT>
+cudaError_t stage_prepare(int k, int mode, int *occ)
 {
-  if constexpr (use_mma<DIM, N, CT>())
+  if constexpr (use_mma<DIM, N, CT>() || use_mma_hanging<DIM, N, CT>())
   {
     using M = MmaShape<N>;
-    const cudaError_t e = occupancy(mma_kernel<N, MODE_STAGE>, M::NT, M::BYTES,
-                                    &occ[MODE_STAGE]);
-    return e != cudaSuccess ? e
-                            : occupancy(mma_kernel<N, MODE_RHS>, M::NT,
-                                        M::BYTES, &occ[MODE_RHS]);
+    if (k == KERNEL_MMA)
+      return prepare_one(mode == MODE_RHS ? mma_kernel<N, MODE_RHS>
+                                          : mma_kernel<N, MODE_STAGE>,
+                         M::NT, M::BYTES, occ);
   }
-  else if constexpr (use_pack<DIM, N, CT>())
+  if constexpr (use_pack<DIM, N, CT>())
   {
     using K = PackShape<DIM, N, CT>;
-    cudaError_t e =
-        allow_smem(dg_pack_kernel<DIM, N, MODE_STAGE_NC, CT>, (int)K::BYTES);
-    if (e == cudaSuccess)
-      e = allow_smem(dg_pack_kernel<DIM, N, MODE_STAGE_CF, CT>, (int)K::BYTES);
-    if (e == cudaSuccess)
-      e = occupancy(dg_pack_kernel<DIM, N, MODE_STAGE, CT>, K::NT, K::BYTES,
-                    &occ[MODE_STAGE]);
-    if (e == cudaSuccess)
-      e = occupancy(dg_pack_kernel<DIM, N, MODE_RHS, CT>, K::NT, K::BYTES,
-                    &occ[MODE_RHS]);
-    if constexpr (pack_has_small<DIM, N>())
-    {
-      const int smem = (int)stage_smem_bytes<DIM, N, CT>();
-      if (e == cudaSuccess)
-        e = allow_smem(single_kernel<DIM, N, CT, MODE_STAGE>, smem);
-      if (e == cudaSuccess)
-        e = allow_smem(single_kernel<DIM, N, CT, MODE_STAGE_NC>, smem);
-      if (e == cudaSuccess)
-        e = allow_smem(
-            single_kernel<DIM, N, CT, conforming_mode<DIM, N, CT>()>, smem);
-      if (e == cudaSuccess)
-        e = allow_smem(single_kernel<DIM, N, CT, MODE_RHS>, smem);
-    }
-    return e;
+    if (k == KERNEL_PACK)
+      return prepare_one(
+          mode == MODE_STAGE      ? pack_kernel<DIM, N, CT, MODE_STAGE>
+          : mode == MODE_STAGE_NC ? pack_kernel<DIM, N, CT, MODE_STAGE_NC>
+          : mode == MODE_STAGE_CF ? pack_kernel<DIM, N, CT, MODE_STAGE_CF>
+                                  : pack_kernel<DIM, N, CT, MODE_RHS>,
+          K::NT, K::BYTES, occ);
   }
+  if constexpr (!use_mma<DIM, N, CT>() &&
+                (!use_pack<DIM, N, CT>() || pack_has_small<DIM, N>()))
+    return prepare_one(
+        mode == MODE_STAGE      ? single_kernel<DIM, N, CT, MODE_STAGE>
+        : mode == MODE_STAGE_NC ? single_kernel<DIM, N, CT, MODE_STAGE_NC>
+        : mode == MODE_STAGE_CF
+            ? single_kernel<DIM, N, CT, conforming_mode<DIM, N, CT>()>
+            : single_kernel<DIM, N, CT, MODE_RHS>,
+        Shape<DIM, N>::NT, stage_smem_bytes<DIM, N, CT>(), occ);
   else
-  {
-    using S = Shape<DIM, N>;
-    const size_t smem = stage_smem_bytes<DIM, N, CT>();
-    cudaError_t e = allow_smem(single_kernel<DIM, N, CT, MODE_STAGE_NC>, (int)smem);
-    if (e == cudaSuccess)
-      e = allow_smem(single_kernel<DIM, N, CT, conforming_mode<DIM, N, CT>()>,
-                     (int)smem);
-    if constexpr (use_mma_hanging<DIM, N, CT>())
-    {
-      // as many resident CTAs in both kernels (MmaShape::MINB), so one
-      // lookahead serves them
-      if (e == cudaSuccess)
-        e = allow_smem(mma_kernel<N, MODE_STAGE>, (int)MmaShape<N>::BYTES);
-      if (e == cudaSuccess)
-        e = allow_smem(mma_kernel<N, MODE_RHS>, (int)MmaShape<N>::BYTES);
-    }
-    if (e == cudaSuccess)
-      e = occupancy(single_kernel<DIM, N, CT, MODE_STAGE>, S::NT, smem,
-                    &occ[MODE_STAGE]);
-    if (e == cudaSuccess)
-      e = occupancy(single_kernel<DIM, N, CT, MODE_RHS>, S::NT, smem,
-                    &occ[MODE_RHS]);
-    return e;
-  }
+    return cudaErrorInvalidDeviceFunction;
 }
 
 template <int DIM, int N, typename CT> KernelSet make_set()
@@ -214,6 +212,7 @@ template <int DIM, int N, typename CT> KernelSet make_set()
   using S = Shape<DIM, N>;
   KernelSet k;
   k.launch = stage_launch<DIM, N, CT>;
+  k.kernel = stage_kernel<DIM, N, CT>;
   k.prepare = stage_prepare<DIM, N, CT>;
   k.energy = dg_energy_kernel<DIM, N>;
   k.NT = S::NT;
@@ -449,6 +448,47 @@ DomainView view(bfam_gpu_domain_t *d, int in)
   return v;
 }
 
+// elements of launch level l
+int level_size(const bfam_gpu_domain_t *d, int l)
+{
+  return d->nlevels > 1 ? d->level_off[l + 1] - d->level_off[l] : d->K;
+}
+
+// The stage mode of launch level l: the first level has no coarse-side faces
+// (unless faces glued to another domain, which are lifted like them, sit
+// there), and a mesh of one level no hanging ones.
+int level_mode(const bfam_gpu_domain_t *d, int l)
+{
+  return l > 0 || d->nglued ? MODE_STAGE
+         : d->nlevels == 1  ? MODE_STAGE_CF
+                            : MODE_STAGE_NC;
+}
+
+// Set-up of the kernel that serves a launch of n elements in a mode, once per
+// domain; which kernel it is in *k.
+cudaError_t prepare_launch(bfam_gpu_domain_t *d, int n, int mode, int *k)
+{
+  *k = d->ks.kernel(n, d->hops.data(), d->sms, mode);
+  int &occ = d->ks.occ[*k][mode];
+  if (occ)
+    return cudaSuccess;
+  const cudaError_t e = d->ks.prepare(*k, mode, &occ);
+  return e == cudaSuccess && occ < 1 ? cudaErrorInvalidConfiguration : e;
+}
+
+int launch_elements(bfam_gpu_domain_t *d, const DomainView &v, int n,
+                    StageParams sp, int mode, cudaStream_t stream, bool overlap)
+{
+  int k;
+  CUDA_TRY(prepare_launch(d, n, mode, &k));
+  // prefetch part of a wave of resident CTAs ahead (half a wave: about half a
+  // CTA lifetime before the element's CTA starts)
+  sp.ahead = d->ks.occ[k][mode] * d->sms *
+             (k == KERNEL_PACK ? d->ks.elements : 1) / d->ks.lookahead;
+  CUDA_TRY(d->ks.launch(v, n, sp, d->hops.data(), mode, stream, overlap));
+  return 0;
+}
+
 int launch_stage(bfam_gpu_domain_t *d, int in, double A, double B, double C,
                  double dt, int first, int mode)
 {
@@ -459,28 +499,18 @@ int launch_stage(bfam_gpu_domain_t *d, int in, double A, double B, double C,
   sp.C = C;
   sp.first_stage = first;
   sp.flux = d->flux;
-  // prefetch part of a wave of resident CTAs ahead (half a wave: about half a
-  // CTA lifetime before the element's CTA starts)
-  sp.ahead = d->ks.occ[mode] * d->sms * d->ks.elements / d->ks.lookahead;
   sp.sms = d->sms;
   DomainView v = view(d, in);
   v.dt = dt;
   // one launch per level; level l's elements after level l-1's
   for (int l = 0; l < d->nlevels; ++l)
   {
-    int n = d->K;
+    const int n = level_size(d, l);
     if (d->nlevels > 1)
-    {
       v.elist = d->elist + d->level_off[l];
-      n = d->level_off[l + 1] - d->level_off[l];
-    }
     if (n == 0)
       continue;
-    // the first level has no coarse-side faces (unless faces glued to
-    // another domain, which are lifted like them, sit there)
-    const int m = mode != MODE_STAGE || l > 0 || d->nglued ? mode
-                  : d->nlevels == 1                         ? MODE_STAGE_CF
-                                                            : MODE_STAGE_NC;
+    const int m = mode == MODE_STAGE ? level_mode(d, l) : mode;
     bfam_gpu_domain::ProfLaunch pl{};
     if (d->prof)
     {
@@ -502,8 +532,8 @@ int launch_stage(bfam_gpu_domain_t *d, int in, double A, double B, double C,
       pl.bytes = per_dof * (double)n * d->Np * d->NFLD;
       CUDA_TRY(cudaEventRecord(pl.t0, d->stream));
     }
-    CUDA_TRY(d->ks.launch(v, n, sp, d->hops.data(), m, d->stream,
-                           true));
+    if (int rc = launch_elements(d, v, n, sp, m, d->stream, true))
+      return rc;
     g_launches.fetch_add(1, std::memory_order_relaxed);
     if (d->prof)
     {
@@ -610,6 +640,8 @@ int bfam_gpu_record_error(int code, const char *msg)
 }
 
 uint64_t bfam_gpu_launch_count(void) { return g_launches.load(); }
+
+uint64_t bfam_gpu_prepare_count(void) { return g_prepares.load(); }
 
 static int create_domain(const bfam_gpu_volume_t *vol,
                          const bfam_gpu_glue_t *glue,
@@ -1119,6 +1151,19 @@ static int create_domain(const bfam_gpu_volume_t *vol,
   d->precision = opts->precision;
   d->device = opts->device;
   d->budget = opts->mem_budget_bytes;
+  d->hops = ops;
+  d->nlevels = nlevels;
+  d->level_off = level_off;
+  // boundary list (glued faces are joined to other domains later)
+  d->bslot = bslot;
+  d->bE.resize(nbnd);
+  d->bF.resize(nbnd);
+  for (int32_t b = 0; b < nbnd; ++b)
+  {
+    d->bE[b] = bnd->EToE[b];
+    d->bF[b] = bnd->EToF[b];
+    d->nglued += bslot[b] >= 0;
+  }
   int rc = 0;
 #define TRY(x)                                                                 \
   do                                                                           \
@@ -1147,12 +1192,17 @@ static int create_domain(const bfam_gpu_volume_t *vol,
       return fail(BFAM_GPU_ECUDA, "stream: %s", cudaGetErrorString(ce));
     }
     d->own_stream = true;
-    ce = ks.prepare(d->ks.occ);
-    if (ce == cudaSuccess && (d->ks.occ[0] < 1 || d->ks.occ[1] < 1))
-      ce = cudaErrorInvalidConfiguration;
-    if (ce == cudaSuccess)
-      ce = cudaDeviceGetAttribute(&d->sms, cudaDevAttrMultiProcessorCount,
-                                  d->device);
+    ce = cudaDeviceGetAttribute(&d->sms, cudaDevAttrMultiProcessorCount,
+                                d->device);
+    // the kernels that this mesh's stages launch (that of the right-hand side
+    // alone: at its first call); set-up loads a kernel, 0.05 ms each (the
+    // first conforming domain of 3D order 2 1.5 ms with all eight of its
+    // shape's kernels, 1.0 with the one that it launches)
+    for (int l = 0; l < d->nlevels && ce == cudaSuccess; ++l)
+    {
+      int k;
+      ce = prepare_launch(d, level_size(d, l), level_mode(d, l), &k);
+    }
     if (ce != cudaSuccess)
     {
       release(d);
@@ -1160,7 +1210,6 @@ static int create_domain(const bfam_gpu_volume_t *vol,
                   cudaGetErrorString(ce));
     }
   }
-  d->hops = ops;
   const size_t state = (size_t)NFLD * d->fs * sizeof(double);
   TRY(dev_alloc(d, (void **)&d->q[0], state));
   TRY(dev_alloc(d, (void **)&d->q[1], state));
@@ -1181,8 +1230,6 @@ static int create_domain(const bfam_gpu_volume_t *vol,
       return fail(BFAM_GPU_ECUDA, "mortar buffer memset failed");
     }
   }
-  d->nlevels = nlevels;
-  d->level_off = level_off;
   if (nlevels > 1)
     TRY(upload(d, &d->elist, elist.data(), elist.size()));
   d->helist = elist;
@@ -1223,16 +1270,6 @@ static int create_domain(const bfam_gpu_volume_t *vol,
   {
     d->hx0.assign(vol->x0, vol->x0 + 3 * (size_t)vol->K);
     d->hh.assign(vol->h, vol->h + 3 * (size_t)vol->K);
-  }
-  // boundary list (glued faces are joined to other domains later)
-  d->bslot = bslot;
-  d->bE.resize(nbnd);
-  d->bF.resize(nbnd);
-  for (int32_t b = 0; b < nbnd; ++b)
-  {
-    d->bE[b] = bnd->EToE[b];
-    d->bF[b] = bnd->EToF[b];
-    d->nglued += bslot[b] >= 0;
   }
   d->hr.assign(vol->r, vol->r + d->Nq);
   d->hw.assign(vol->w, vol->w + d->Nq);

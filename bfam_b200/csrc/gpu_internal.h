@@ -18,6 +18,8 @@ namespace host
 int fail(int code, const char *fmt, ...);
 // kernels launched by the library (bfam_gpu_launch_count)
 extern std::atomic<uint64_t> g_launches;
+// stage kernels set up for launching (bfam_gpu_prepare_count)
+extern std::atomic<uint64_t> g_prepares;
 
 #define CUDA_TRY(call)                                                         \
   do                                                                           \
@@ -55,23 +57,36 @@ cudaError_t launch_dependent(bool overlap, void (*kernel)(P...), dim3 grid,
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
-// per-order launchers (the kernels' parameter lists depend on the order)
+// the kernels that serve the shapes: a thread per node, several elements per
+// CTA, the matrix instruction
+enum
+{
+  KERNEL_NODE = 0,
+  KERNEL_PACK = 1,
+  KERNEL_MMA = 2
+};
+
+// per-order launchers (the kernels' parameter lists depend on the order);
+// which kernel serves a launch of n elements, and its set-up: shared-memory
+// opt-in, resident CTAs per SM
 typedef cudaError_t (*stage_launch_fn)(const DomainView &, int n,
                                 const StageParams &, const double *D,
                                 int mode, cudaStream_t, bool overlap);
-typedef cudaError_t (*prepare_fn)(int *occ);
+typedef int (*stage_kernel_fn)(int n, const double *hops, int sms, int mode);
+typedef cudaError_t (*prepare_fn)(int kernel, int mode, int *occ);
 typedef void (*energy_fn)(const double *, size_t, const ElemData *,
                           const double *, double *);
 
 struct KernelSet
 {
   stage_launch_fn launch = nullptr;
+  stage_kernel_fn kernel = nullptr;
   prepare_fn prepare = nullptr;
   energy_fn energy = nullptr;
   int NT = 0;
-  int occ[2] = {0, 0}; // resident CTAs per SM of the stage and rhs kernels
-  int elements = 1;    // elements per CTA
-  int lookahead = 2;   // L2 lookahead: that part of a wave of resident CTAs
+  int occ[3][4] = {}; // resident CTAs per SM by kernel and mode (0: not set up)
+  int elements = 1;   // elements per CTA of the packed kernel
+  int lookahead = 2;  // L2 lookahead: that part of a wave of resident CTAs
 };
 
 // the kernels of one (dim, order, precision)
@@ -209,6 +224,9 @@ int upload(bfam_gpu_domain_t *d, T **dst, const T *src, size_t n)
 
 // the stage kernel's view of a domain whose stage input is q[in]
 DomainView view(bfam_gpu_domain_t *d, int in);
+// one launch over n elements of v, the domain's view
+int launch_elements(bfam_gpu_domain_t *d, const DomainView &v, int n,
+                    StageParams sp, int mode, cudaStream_t stream, bool overlap);
 int launch_stage(bfam_gpu_domain_t *d, int in, double A, double B, double C,
                  double dt, int first, int mode);
 

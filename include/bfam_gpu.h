@@ -445,6 +445,11 @@ int bfam_gpu_batch_set_tile(bfam_gpu_batch_t *b, int g, int tile,
 
 /* Kernel launches issued by this library since process start. */
 uint64_t bfam_gpu_launch_count(void);
+/* Stage kernels set up for launching (shared-memory opt-in, occupancy; a
+ * kernel is loaded by it) since process start: creating a domain or batch sets
+ * up those that its stages launch, the first bfam_gpu_domain_rhs that of the
+ * right-hand side. */
+uint64_t bfam_gpu_prepare_count(void);
 
 /* Copy of the last error message of the calling thread (NUL-terminated,
  * truncated to len). Returns the message length. */
