@@ -97,7 +97,10 @@ struct TileImpl
   {
     const DiffOp<N, CT> dop = make_diffop<N, CT>(hops);
     return launch_dependent(overlap, kernel<MODE>, grid, NT * EPC, SMEM, st, v,
-                            w, nwork, sp, dop);
+                            w, nwork,
+                            with_early((sp.widest + EPC - 1) / EPC, sp,
+                                       late_from<DIM, N, CT>()),
+                            dop);
   }
   static auto of(int mode)
   {
@@ -149,7 +152,11 @@ template <int DIM, int N, typename CT> struct PackTile
     const StageParams pp = pack_params<DIM, N, K::E>(nwork, sp);
     return launch_dependent(overlap, dg_pack_batch_kernel<DIM, N, MODE, CT>,
                             pack_ctas(nwork, pp), K::NT, K::BYTES, st, v, w,
-                            nwork, pp, dop);
+                            nwork,
+                            with_early(pack_ctas(sp.widest, pack_params<DIM, N, K::E>(
+                                                                sp.widest, sp)),
+                                       pp, pack_late_from<DIM, N, CT>()),
+                            dop);
   }
   static auto of(int mode)
   {
@@ -202,7 +209,8 @@ template <int N, int MINB> struct MmaTile
                      const StageParams &sp, const double *hops, int grid,
                      cudaStream_t st, bool overlap)
   {
-    return launch_dependent(overlap, kernel, grid, M::NT, M::BYTES, st, v, w, nwork, sp,
+    return launch_dependent(overlap, kernel, grid, M::NT, M::BYTES, st, v, w, nwork,
+                            with_early(sp.widest, sp, MMA_LATE_FROM),
                             1.0 / hops[7 * (N + 1) * (N + 1)]);
   }
   static cudaError_t prepare(int, int, int)
@@ -448,7 +456,9 @@ struct bfam_gpu_batch
     std::vector<int2 *> work;
     std::vector<int64_t> nwork_l;
     std::vector<int> grid;
-    int ahead = 0; // L2 prefetch distance of one-buffer tiles (work items)
+    int ahead = 0; // L2 prefetch distance (work items)
+    int slots = 0;  // resident CTAs of the tile's kernel
+    int widest = 0; // work items of the largest level
     // no domain of the group has faces glued to another order, so level 0
     // holds no element with a coarse-side face (launched without that pass)
     bool level0_nc = false;
@@ -584,6 +594,7 @@ int choose_grid(bfam_gpu_batch_t *b, bfam_gpu_batch_t::Group &g)
   // L2 lookahead in work items
   const int epc = t.pack ? t.pack : t.EPC;
   g.ahead = (int)std::min<int64_t>(full * epc / t.lookahead, INT32_MAX);
+  g.slots = occ * b->sms;
   g.grid.resize(g.nwork_l.size());
   for (size_t l = 0; l < g.nwork_l.size(); ++l)
     g.grid[l] = (int)((g.nwork_l[l] + t.EPC - 1) / t.EPC);
@@ -689,6 +700,8 @@ int issue_step(bfam_gpu_batch_t *b, int p)
       sp.flux = g.flux;
       sp.ahead = g.ahead;
       sp.sms = b->sms;
+      sp.slots = g.slots;
+      sp.widest = g.widest;
       // levels in order: coarse elements after the fine ones across their
       // hanging faces
       for (size_t l = 0; l < g.work.size(); ++l)
@@ -780,6 +793,8 @@ int issue_step_glued(bfam_gpu_batch_t *b, int p)
       sp.flux = g.flux;
       sp.ahead = g.ahead;
       sp.sms = b->sms;
+      sp.slots = g.slots;
+      sp.widest = g.widest;
       for (size_t l = 0; l < g.work.size(); ++l)
       {
         if (int rc = launch_level(b, g, l, par, sp, st, false))
@@ -1127,6 +1142,7 @@ int bfam_gpu_batch_create(bfam_gpu_domain_t *const *doms, int ndom,
                       cudaMemcpyHostToDevice));
       G.work.push_back(dw);
       G.nwork_l.push_back((int64_t)work.size());
+      G.widest = std::max(G.widest, (int)work.size());
     }
     for (int p = 0; p < 2; ++p)
       TRY(batch_alloc(b, (void **)&G.views[p],

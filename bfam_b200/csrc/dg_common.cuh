@@ -84,7 +84,10 @@ struct StageParams
   // its loads find L2 (0: no prefetch)
   int ahead;
   int sms;     // SMs of the device
-  int per = 0; // packed kernel: elements per CTA, set by its launch
+  int widest = 0; // elements of the stage's largest launch
+  int slots = 0;  // resident CTAs of the kernel on the device
+  int per = 0;   // packed kernel: elements per CTA, set by its launch
+  int early = 1; // the next launch's CTAs may start before this one's end
 };
 
 // Ricker wavelet (1 - 2 a) exp(-a), a = (pi f0 (t - t0))^2

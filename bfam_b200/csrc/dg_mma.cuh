@@ -89,6 +89,11 @@ __host__ __device__ constexpr bool use_mma_hanging()
 {
   return DIM == 3 && N == 5 && sizeof(CT) == sizeof(double);
 }
+// as late_from: N = 5, 331 elements with hanging faces (262 of them, 0.35, in the
+// first launch) 76.2 us per step early and 72.3 late, 204 69.1 and 71.3; N = 6,
+// 256 (0.58) 59.9 and 46.6
+constexpr int MMA_LATE_FROM = 34;
+
 // hops: the domain's operators Dr | interpolation[3] | projection[3] | w; a
 // domain without a glue grid has identities for interpolations
 template <int N> inline bool mma_for_mesh(const double *hops)
@@ -460,7 +465,8 @@ __device__ __forceinline__ void mma_element(const Item &item, int n,
   const double2 fx = make_double2(dfrag(2 * c), dfrag(2 * c + 1));
   const double2 fy = YS ? make_double2(dfrag(c), dfrag(c + 4)) : fx;
   __syncthreads();
-  grid_launch_dependents(); // as in dg_stage.cuh, not earlier
+  if (sp.early)
+    grid_launch_dependents(); // as in dg_stage.cuh, not earlier
   const double a = MODE != MODE_RHS ? sp.A : 0.0;
   const double s = MODE != MODE_RHS ? d.dt : 1.0;
   const int n0 = w * P + r * Nq + i0, m0 = n0 + w * (PP - P);

@@ -110,6 +110,15 @@ template <int DIM, int N> bool pack_too_small(int n, int sms, int mode)
   return pack_has_small<DIM, N>() && n < (mode == MODE_STAGE_CF ? 12 : 48) * sms;
 }
 
+// As late_from: the plain form's launches at 3D N = 2 are long enough to wait for
+// (2,744 conforming elements, 0.58 of a wave, 60.7 us per step early and 53.4
+// late; in the precision form 45.9 and 47.5), others not (3D N = 1, 1,000 16.8
+// and 17.8).
+template <int DIM, int N, typename CT> constexpr int pack_late_from()
+{
+  return DIM == 3 && N == 2 && sizeof(CT) == sizeof(double) ? 50 : 85;
+}
+
 // The 1-D mortar pass of line_apply on `lines` faces of NC fields each (2D
 // orders 6 and up), a thread per value instead of per line: a CTA has few
 // lines there, and a thread per line left most of it waiting for Nq x Nq
@@ -427,7 +436,8 @@ __device__ __forceinline__ void pack_elements(const Item &item, int n,
     }
   }
   __syncthreads();
-  grid_launch_dependents(); // as in dg_stage.cuh, not earlier
+  if (sp.early)
+    grid_launch_dependents(); // as in dg_stage.cuh, not earlier
   if (!mine)
     return;
 
