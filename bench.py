@@ -599,14 +599,17 @@ def run_serving(args):
     from oracle import oracle as orc
 
     prec = bf.PRECISION_FP64 if args.precision == "fp64" else bf.PRECISION_FP32
-    # tile choices for the request orders, before any clock starts
-    for N in (3, 5):
+    # tile choices for the request orders, one request alone and several,
+    # before any clock starts
+    for N, count in ((3, 1), (3, 2), (5, 1), (5, 2)):
         m = bf.Mesh(3, N, (8, 8, 8))
-        d = bf.GpuDomain(m, 1.0, 2.0, 1.0, precision=prec, device=local)
-        b = bf.Batch([d])
+        ds = [bf.GpuDomain(m, 1.0, 2.0, 1.0, precision=prec, device=local)
+              for _ in range(count)]
+        b = bf.Batch(ds)
         autotune.autotune(b, device=local)
         b.free()
-        d.free()
+        for d in ds:
+            d.free()
     runs = []
     checks = []
     n0 = bf.launch_count()

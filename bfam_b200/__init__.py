@@ -180,6 +180,7 @@ def _declare(L: C.CDLL) -> None:
         "bfam_gpu_tile_shape": (C.c_int, [C.c_int, C.c_int, C.c_int, P(C.c_int),
                                           P(C.c_int)]),
         "bfam_gpu_batch_set_tile": (C.c_int, [vp, C.c_int, C.c_int, C.c_int]),
+        "bfam_gpu_batch_group_mesh": (C.c_int, [vp, C.c_int, P(C.c_int), P(C.c_int)]),
         "bfam_gpu_launch_count": (C.c_uint64, []),
         "bfam_gpu_prepare_count": (C.c_uint64, []),
         "bfam_gpu_last_error": (C.c_int, [C.c_char_p, C.c_size_t]),
@@ -682,8 +683,10 @@ class Batch:
             d, n, p, k = C.c_int(), C.c_int(), C.c_int(), C.c_int64()
             _check(L.bfam_gpu_batch_group_info(self._h, g, C.byref(d), C.byref(n),
                                                C.byref(p), C.byref(k)))
+            nd, h = C.c_int(), C.c_int()
+            _check(L.bfam_gpu_batch_group_mesh(self._h, g, C.byref(nd), C.byref(h)))
             out.append({"dim": d.value, "N": n.value, "precision": p.value,
-                        "elements": k.value})
+                        "elements": k.value, "domains": nd.value, "hanging": bool(h.value)})
         return out
 
     def launches_per_step(self) -> int:

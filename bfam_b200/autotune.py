@@ -4,11 +4,14 @@ A batch runs one launch per order group, level and LSRK stage.  The tile of a
 group is (elements per CTA, threads per element, register budget for a
 number of resident CTAs per SM), chosen among the shapes compiled for that
 order (`tile_shapes`, `tile_elements`), plus the CTAs per SM of the L2
-lookahead distance.  The tuner times every candidate on a synthetic domain of the group's order, precision and
-roughly its element count (a 20 % refined brick, Gaussian pulse, random
-material, capped in size so tuning takes seconds), with CUDA events on the
-batch's stream over a few graph-replayed steps, and keeps the fastest.
-Results are cached per GPU name in a JSON file.
+lookahead distance.  The tuner times every candidate on a synthetic group that
+runs the same kernels: of the group's order and precision, roughly its element
+count, on 20 % refined or conforming bricks as the group's meshes have hanging
+faces or not, and of one domain or two as the group has one or several (a group
+of one under the default tile runs the single-domain kernel; Gaussian pulse,
+random material, capped in size so tuning takes seconds).  It times with CUDA
+events on the batch's stream over a few graph-replayed steps and keeps the
+fastest.  Results are cached per GPU name in a JSON file.
 """
 from __future__ import annotations
 
@@ -33,14 +36,17 @@ def _brick_for(dim: int, elements: int, refine_prob: float = 0.2):
     return (n,) * dim
 
 
-def _key(gpu: str, dim: int, N: int, precision: int) -> str:
-    """cache key: the GPU, the group, and the library's tile table for the
-    order (threads x register budget x elements per CTA of every tile), so
-    that a library with another table never reuses a tile index chosen
-    against the old one"""
+def _key(gpu: str, dim: int, N: int, precision: int, hanging: bool = True,
+         domains: int = 1) -> str:
+    """cache key: the GPU, the group (order, precision, kind of mesh, one
+    domain or several), and the library's tile table for the order (threads x
+    register budget x elements per CTA of every tile), so that a library with
+    another table never reuses a tile index chosen against the old one"""
     table = "-".join(f"{t}x{m}x{e}" for (t, m), e in
                      zip(tile_shapes(dim, N), tile_elements(dim, N)))
-    return f"{gpu}|dim{dim}|N{N}|prec{precision}|tiles:{table}"
+    return (f"{gpu}|dim{dim}|N{N}|prec{precision}|tiles:{table}"
+            f"|mesh:{'hanging' if hanging else 'conforming'}"
+            f"|domains:{'one' if domains == 1 else 'several'}")
 
 
 def load_cache(path: Path | None = None) -> dict:
@@ -57,21 +63,28 @@ def save_cache(cache: dict, path: Path | None = None) -> None:
 
 
 def tune_group(dim: int, N: int, precision: int, elements: int, steps: int = 4,
-               device: int = 0, seed: int = 5) -> dict:
+               device: int = 0, seed: int = 5, hanging: bool = True,
+               domains: int = 1) -> dict:
     """Time every (tile, CTAs per SM) candidate; returns the table and the best."""
     import torch
 
-    n = _brick_for(dim, min(elements, MAX_TUNE_ELEMENTS))
-    mesh = Mesh(dim, N, n, refine_prob=0.2, seed=seed)
-    rho, lam, mu = material_random(mesh.K, seed)
-    r = lgl_operators(N)[0]
-    q0 = mesh.gaussian_pulse(r, (0.5, 0.5, 0.5), 0.1)
-    cp = np.sqrt((lam + 2 * mu) / rho)
-    dt = 0.3 * float(np.min(mesh.h[:, :dim].min(axis=1) / cp)) / (N * N)
-    dom = GpuDomain(mesh, rho, lam, mu, precision=precision, device=device)
-    dom.set_fields(q0)
+    p = 0.2 if hanging else 0.0
+    count = 1 if domains == 1 else 2
+    n = _brick_for(dim, min(elements, MAX_TUNE_ELEMENTS) // count, p)
+    doms, dts, total, ndof = [], [], 0, 0
+    for k in range(count):
+        mesh = Mesh(dim, N, n, refine_prob=p, seed=seed + k)
+        rho, lam, mu = material_random(mesh.K, seed + k)
+        r = lgl_operators(N)[0]
+        cp = np.sqrt((lam + 2 * mu) / rho)
+        dts.append(0.3 * float(np.min(mesh.h[:, :dim].min(axis=1) / cp)) / (N * N))
+        dom = GpuDomain(mesh, rho, lam, mu, precision=precision, device=device)
+        dom.set_fields(mesh.gaussian_pulse(r, (0.5, 0.5, 0.5), 0.1))
+        doms.append(dom)
+        total += mesh.K
+        ndof += mesh.ndof
     stream = torch.cuda.Stream(device=device)
-    b = Batch([dom])
+    b = Batch(doms)
     b.set_stream(stream.cuda_stream)
     table = []
     shapes = tile_shapes(dim, N)
@@ -82,22 +95,23 @@ def tune_group(dim: int, N: int, precision: int, elements: int, steps: int = 4,
                 b.set_tile(0, tile, cps)
             except BfamGpuError:
                 continue  # does not fit an SM on this device
-            b.step([dt], 1)  # capture + warm-up
+            b.step(dts, 1)  # capture + warm-up
             e0 = torch.cuda.Event(enable_timing=True)
             e1 = torch.cuda.Event(enable_timing=True)
             e0.record(stream)
-            b.step([dt], steps)
+            b.step(dts, steps)
             e1.record(stream)
             e1.synchronize()
             ms = e0.elapsed_time(e1) / steps
             table.append({"tile": tile, "threads": threads, "elements_per_cta": epc,
                           "min_ctas": minb, "ctas_per_sm": cps, "ms_per_step": ms,
-                          "dof_updates_per_s": mesh.ndof * 5 / (ms / 1e3)})
+                          "dof_updates_per_s": ndof * 5 / (ms / 1e3)})
     b.free()
-    dom.free()
+    for dom in doms:
+        dom.free()
     best = min(table, key=lambda t: t["ms_per_step"])
     return {"best": {"tile": best["tile"], "ctas_per_sm": best["ctas_per_sm"]},
-            "elements": mesh.K, "table": table}
+            "elements": total, "table": table}
 
 
 def autotune(batch: Batch, cache: dict | None = None, cache_path=None,
@@ -112,10 +126,11 @@ def autotune(batch: Batch, cache: dict | None = None, cache_path=None,
     choices = []
     dirty = False
     for g, info in enumerate(batch.groups()):
-        key = _key(gpu, info["dim"], info["N"], info["precision"])
+        kind = {"hanging": info["hanging"], "domains": info["domains"]}
+        key = _key(gpu, info["dim"], info["N"], info["precision"], **kind)
         if key not in cache:
             cache[key] = tune_group(info["dim"], info["N"], info["precision"],
-                                    info["elements"], device=device)
+                                    info["elements"], device=device, **kind)
             dirty = True
         best = cache[key]["best"]
         batch.set_tile(g, best["tile"], best["ctas_per_sm"])

@@ -313,7 +313,7 @@ std::vector<BatchTile> tiles(int dim, int N, int precision,
                              const double *hops = nullptr)
 {
   if (dim == 3 && precision != BFAM_GPU_PRECISION_FP32 &&
-      (N == 6 || N == 7 || (N == 5 && hops && mma_for_mesh<5>(hops))))
+      (N == 6 || N == 7 || (N == 5 && hops && mesh_hangs(hops, 5))))
     return mma_tiles(N);
   return precision == BFAM_GPU_PRECISION_FP32 ? tiles_for<float>(dim, N)
                                               : tiles_for<double>(dim, N);
@@ -1085,7 +1085,7 @@ int bfam_gpu_batch_create(bfam_gpu_domain_t *const *doms, int ndom,
       // batch kernel does not spill (104 against 100 G DOF-updates/s)
       G.multi_tile = d->dim == 3 && d->N == 5 &&
                      d->precision == BFAM_GPU_PRECISION_FP64 &&
-                     !mma_for_mesh<5>(d->hops.data());
+                     !mesh_hangs(d->hops.data(), 5);
       if (G.tiles.empty())
       {
         batch_release(b);
@@ -1336,6 +1336,19 @@ int bfam_gpu_batch_group_info(const bfam_gpu_batch_t *b, int g, int *dim,
     *precision = G.precision;
   if (elements)
     *elements = G.nwork;
+  return 0;
+}
+
+int bfam_gpu_batch_group_mesh(const bfam_gpu_batch_t *b, int g, int *domains,
+                              int *hanging)
+{
+  if (!b || g < 0 || g >= (int)b->groups.size())
+    return fail(BFAM_GPU_EINVAL, "no group %d", g);
+  const auto &G = b->groups[g];
+  if (domains)
+    *domains = (int)G.doms.size();
+  if (hanging)
+    *hanging = mesh_hangs(G.hops.data(), G.N);
   return 0;
 }
 

@@ -99,7 +99,7 @@ int stage_kernel(int n, const double *hops, int sms, int mode)
 {
   if constexpr (use_mma_hanging<DIM, N, CT>())
   {
-    if (mma_for_mesh<N>(hops))
+    if (mesh_hangs(hops, N))
       return KERNEL_MMA;
   }
   if constexpr (pack_has_small<DIM, N>())

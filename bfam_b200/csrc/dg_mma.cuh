@@ -76,7 +76,7 @@ template <int N> struct MmaShape
 };
 
 // Orders and arithmetic the kernel serves: always at orders 6 and 7, and at
-// order 5 where the domain's mesh has hanging faces (mma_for_mesh): with 30 %
+// order 5 where the domain's mesh has hanging faces (mesh_hangs): with 30 %
 // of the base cells refined 127 G DOF-updates/s here against 123.5 in the
 // node-per-thread kernel, conforming 155 against 162.
 template <int DIM, int N, typename CT>
@@ -94,11 +94,12 @@ __host__ __device__ constexpr bool use_mma_hanging()
 // 256 (0.58) 59.9 and 46.6
 constexpr int MMA_LATE_FROM = 34;
 
-// hops: the domain's operators Dr | interpolation[3] | projection[3] | w; a
-// domain without a glue grid has identities for interpolations
-template <int N> inline bool mma_for_mesh(const double *hops)
+// hops: an order-N domain's operators Dr | interpolation[3] | projection[3] | w;
+// a domain without a glue grid, so without hanging faces, has identities for
+// interpolations
+inline bool mesh_hangs(const double *hops, int N)
 {
-  constexpr int n = N + 1;
+  const int n = N + 1;
   const double *bottom = hops + 2 * n * n;
   for (int i = 0; i < n * n; ++i)
     if (bottom[i] != (i % (n + 1) == 0 ? 1.0 : 0.0))

@@ -382,6 +382,11 @@ int bfam_gpu_batch_free(bfam_gpu_batch_t *b);
 int bfam_gpu_batch_num_groups(const bfam_gpu_batch_t *b);
 int bfam_gpu_batch_group_info(const bfam_gpu_batch_t *b, int g, int *dim,
                               int *N, int *precision, int64_t *elements);
+/* What else selects the kernels that group g runs: its number of domains (one
+ * under the default tile runs the single-domain kernel) and whether their
+ * meshes have hanging faces (they come with a glue grid's operators). */
+int bfam_gpu_batch_group_mesh(const bfam_gpu_batch_t *b, int g, int *domains,
+                              int *hanging);
 
 /* ------------------------------------------------------------------------
  * Glue between two domains, e.g. of different orders (p-nonconforming
