@@ -176,6 +176,8 @@ def _declare(L: C.CDLL) -> None:
         "bfam_gpu_batch_group_info": (C.c_int, [vp, C.c_int, P(C.c_int), P(C.c_int),
                                                 P(C.c_int), P(C.c_int64)]),
         "bfam_gpu_tile_count": (C.c_int, [C.c_int, C.c_int]),
+        "bfam_gpu_tile_kernel": (C.c_int, [C.c_int] * 5 + [C.c_char_p, C.c_size_t]
+                                 + [P(C.c_int)] * 3),
         "bfam_gpu_tile_elements": (C.c_int, [C.c_int, C.c_int, C.c_int]),
         "bfam_gpu_tile_shape": (C.c_int, [C.c_int, C.c_int, C.c_int, P(C.c_int),
                                           P(C.c_int)]),
@@ -634,6 +636,20 @@ def tile_elements(dim: int, N: int) -> list[int]:
         e = L.bfam_gpu_tile_elements(dim, N, t)
         _check(min(e, 0))
         out.append(int(e))
+    return out
+
+
+def tile_kernels(dim: int, N: int, precision: int, hanging: bool) -> list[tuple]:
+    """(kernel, threads per CTA, resident CTAs per SM, elements per CTA) of every
+    tile in groups of one precision, on meshes with hanging faces or without"""
+    L = lib()
+    out = []
+    for t in range(L.bfam_gpu_tile_count(dim, N)):
+        name = C.create_string_buffer(16)
+        v = [C.c_int() for _ in range(3)]
+        _check(L.bfam_gpu_tile_kernel(dim, N, precision, int(hanging), t, name, len(name),
+                                      *(C.byref(x) for x in v)))
+        out.append((name.value.decode(), *(x.value for x in v)))
     return out
 
 

@@ -23,7 +23,7 @@ from pathlib import Path
 import numpy as np
 
 from . import (Batch, BfamGpuError, GpuDomain, Mesh, lgl_operators, material_random,
-               tile_elements, tile_shapes)
+               tile_elements, tile_kernels, tile_shapes)
 
 DEFAULT_CACHE = Path(__file__).resolve().parent / "tile_cache.json"
 MAX_TUNE_ELEMENTS = 24000
@@ -39,12 +39,14 @@ def _brick_for(dim: int, elements: int, refine_prob: float = 0.2):
 def _key(gpu: str, dim: int, N: int, precision: int, hanging: bool = True,
          domains: int = 1) -> str:
     """cache key: the GPU, the group (order, precision, kind of mesh, one
-    domain or several), and the library's tile table for the order (threads x
-    register budget x elements per CTA of every tile), so that a library with
-    another table never reuses a tile index chosen against the old one"""
+    domain or several), and the library's tiles, as shapes of the order (threads
+    x register budget x elements per CTA) and as the kernels that such a group
+    runs under them, so that a library with other tiles never reuses a tile index
+    chosen against the old ones"""
     table = "-".join(f"{t}x{m}x{e}" for (t, m), e in
                      zip(tile_shapes(dim, N), tile_elements(dim, N)))
-    return (f"{gpu}|dim{dim}|N{N}|prec{precision}|tiles:{table}"
+    kernels = "-".join(".".join(map(str, k)) for k in tile_kernels(dim, N, precision, hanging))
+    return (f"{gpu}|dim{dim}|N{N}|prec{precision}|tiles:{table}|kernels:{kernels}"
             f"|mesh:{'hanging' if hanging else 'conforming'}"
             f"|domains:{'one' if domains == 1 else 'several'}")
 
@@ -87,9 +89,8 @@ def tune_group(dim: int, N: int, precision: int, elements: int, steps: int = 4,
     b = Batch(doms)
     b.set_stream(stream.cuda_stream)
     table = []
-    shapes = tile_shapes(dim, N)
-    epcs = tile_elements(dim, N)
-    for tile, ((threads, minb), epc) in enumerate(zip(shapes, epcs)):
+    for tile, (kernel, threads, minb, epc) in enumerate(
+            tile_kernels(dim, N, precision, hanging)):
         for cps in sorted({0, max(1, minb - 1)} if minb > 1 else {0}):
             try:
                 b.set_tile(0, tile, cps)
@@ -103,7 +104,8 @@ def tune_group(dim: int, N: int, precision: int, elements: int, steps: int = 4,
             e1.record(stream)
             e1.synchronize()
             ms = e0.elapsed_time(e1) / steps
-            table.append({"tile": tile, "threads": threads, "elements_per_cta": epc,
+            table.append({"tile": tile, "kernel": kernel, "threads": threads,
+                          "elements_per_cta": epc,
                           "min_ctas": minb, "ctas_per_sm": cps, "ms_per_step": ms,
                           "dof_updates_per_s": ndof * 5 / (ms / 1e3)})
     b.free()

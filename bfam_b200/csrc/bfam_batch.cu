@@ -19,6 +19,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdio>
 #include <cstring>
 #include <map>
 #include <tuple>
@@ -41,7 +42,12 @@ typedef int (*batch_occupancy_fn)(int mode);
 
 struct BatchTile
 {
+  // shape as reported to callers (bfam_gpu_tile_shape): threads per element,
+  // CTAs per SM that the register budget is for
   int NT = 0, MINB = 0;
+  // the kernel that runs: its name, threads and budget of a CTA
+  const char *kernel = "node";
+  int threads = 0, budget = 0;
   int lookahead = 2; // L2 lookahead: that part of a wave of resident CTAs
   int EPC = 1; // elements per CTA (NT threads each)
   int pack = 0; // elements per CTA of the packed kernel (0: not packed)
@@ -119,6 +125,8 @@ struct TileImpl
     t.NT = NT;
     t.MINB = MINB;
     t.EPC = EPC;
+    t.threads = NT * EPC;
+    t.budget = MINB;
     t.launch = run<MODE_STAGE>;
     t.launch_nc = run<MODE_STAGE_NC>;
     t.launch_cf = run<conforming_mode<DIM, N, CT>()>;
@@ -180,6 +188,9 @@ template <int DIM, int N, typename CT> struct PackTile
     t.NT = Shape<DIM, N>::NT;
     t.MINB = stage_min_ctas<DIM, N, CT>();
     t.pack = K::E;
+    t.kernel = "pack";
+    t.threads = K::NT;
+    t.budget = K::MINB;
     t.launch = run<MODE_STAGE>;
     t.launch_nc = run<MODE_STAGE_NC>;
     t.launch_cf = run<MODE_STAGE_CF>;
@@ -223,6 +234,9 @@ template <int N, int MINB> struct MmaTile
     BatchTile t;
     t.NT = M::NT;
     t.MINB = MINB;
+    t.kernel = "mma";
+    t.threads = M::NT;
+    t.budget = MINB;
     t.lookahead = N == 7 ? 4 : 2; // as for single domains
     t.launch = t.launch_nc = t.launch_cf = launch;
     t.prepare = prepare;
@@ -295,38 +309,41 @@ template <typename CT> std::vector<BatchTile> tiles_for(int dim, int N)
   return v;
 }
 
-// the plain form's tiles under the matrix kernel, as many as the precision
-// form has: one kernel under several register budgets
+// the plain form's tiles under the matrix kernel: one kernel under the register
+// budgets for 1 to MINB resident CTAs per SM and, at N = 5, one more, the
+// single-domain kernel's first (two refined domains at N = 5, 5, 4, 3, 1, 2 and 6
+// CTAs: 116, 121, 110, 111, 111 and 98 G DOF-updates/s)
 std::vector<BatchTile> mma_tiles(int N)
 {
   if (N == 5)
     return {MmaTile<5, MmaShape<5>::MINB>::make(), MmaTile<5, 4>::make(),
             MmaTile<5, 3>::make(),                 MmaTile<5, 1>::make(),
-            MmaTile<5, 2>::make(),                 MmaTile<5, 2>::make()};
+            MmaTile<5, 2>::make(),                 MmaTile<5, 6>::make()};
   if (N == 6)
     return {MmaTile<6, MmaShape<6>::MINB>::make()};
   return {MmaTile<7, MmaShape<7>::MINB>::make(), MmaTile<7, 1>::make()};
 }
 
-// hops: the group's operators (the node-per-thread kernel's table without)
-std::vector<BatchTile> tiles(int dim, int N, int precision,
-                             const double *hops = nullptr)
+// A group's tiles.  hanging: its operators come from meshes with hanging faces.
+std::vector<BatchTile> tiles(int dim, int N, int precision, bool hanging)
 {
   if (dim == 3 && precision != BFAM_GPU_PRECISION_FP32 &&
-      (N == 6 || N == 7 || (N == 5 && hops && mesh_hangs(hops, 5))))
+      (N == 6 || N == 7 || (N == 5 && hanging)))
     return mma_tiles(N);
   return precision == BFAM_GPU_PRECISION_FP32 ? tiles_for<float>(dim, N)
                                               : tiles_for<double>(dim, N);
 }
 
-// The table that describes an order's tiles to callers: the plain form's, and
-// at 3D orders 6 and 7, where the plain form's tiles are the matrix
-// kernel's, the precision form's (one thread per face node at least).
+// The shapes of an order's tiles, the same for every group of the order: the
+// node-per-thread kernel's on conforming meshes, of the precision form at 3D
+// orders 6 and 7, where the plain form's tiles are the matrix kernel's.  What a
+// group runs is in tiles() (bfam_gpu_tile_kernel).
 std::vector<BatchTile> shape_table(int dim, int N)
 {
-  return dim == 3 && (N == 6 || N == 7)
-             ? tiles(dim, N, BFAM_GPU_PRECISION_FP32)
-             : tiles(dim, N, BFAM_GPU_PRECISION_FP64);
+  return tiles(dim, N,
+               dim == 3 && (N == 6 || N == 7) ? BFAM_GPU_PRECISION_FP32
+                                              : BFAM_GPU_PRECISION_FP64,
+               false);
 }
 
 // ----------------------------------------------------- point location
@@ -996,6 +1013,25 @@ int bfam_gpu_tile_elements(int dim, int N, int tile)
   return t[tile].EPC;
 }
 
+int bfam_gpu_tile_kernel(int dim, int N, int precision, int hanging, int tile,
+                         char *name, size_t len, int *threads, int *min_ctas,
+                         int *elements)
+{
+  const auto t = tiles(dim, N, precision, hanging != 0);
+  if (tile < 0 || tile >= (int)t.size())
+    return fail(BFAM_GPU_EINVAL, "no tile %d for dim %d order %d", tile, dim,
+                N);
+  if (name && len)
+    std::snprintf(name, len, "%s", t[tile].kernel);
+  if (threads)
+    *threads = t[tile].threads;
+  if (min_ctas)
+    *min_ctas = t[tile].budget;
+  if (elements)
+    *elements = t[tile].pack ? t[tile].pack : t[tile].EPC;
+  return 0;
+}
+
 // ---------------------------------------------------------------- batch
 
 int bfam_gpu_batch_create(bfam_gpu_domain_t *const *doms, int ndom,
@@ -1080,7 +1116,8 @@ int bfam_gpu_batch_create(bfam_gpu_domain_t *const *doms, int ndom,
       G.precision = d->precision;
       G.flux = d->flux;
       G.hops = d->hops;
-      G.tiles = tiles(d->dim, d->N, d->precision, d->hops.data());
+      G.tiles = tiles(d->dim, d->N, d->precision,
+                      mesh_hangs(d->hops.data(), d->N));
       // several conforming domains at N = 5 in FP64: the four-CTA tile, whose
       // batch kernel does not spill (104 against 100 G DOF-updates/s)
       G.multi_tile = d->dim == 3 && d->N == 5 &&

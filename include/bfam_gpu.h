@@ -429,20 +429,32 @@ int bfam_gpu_pglue_free(bfam_gpu_pglue_t *g);
  * added glue when the batch steps. */
 int bfam_gpu_batch_add_pglue(bfam_gpu_batch_t *b, bfam_gpu_pglue_t *g);
 
-/* Tile shapes compiled for an order: tile t runs bfam_gpu_tile_elements
- * elements per CTA with `threads` threads each (a tile with fewer threads
- * than nodes or face nodes loops over them; each element of a CTA has its
- * own shared-memory tile and barrier, down to one warp per element) and a
- * register budget for `min_ctas` resident CTAs per SM.  Tile 0 is the
- * single-domain kernel's (one element per CTA).  At 3D orders 6 and 7 the
- * shapes are the precision form's; the plain form's tiles there are one warp
- * per plane of nodes.  In 2D and at 3D orders 1 and 2 tile 0 packs several
- * elements into a CTA, a thread per node, whatever shape it reports. */
+/* Tile shapes of an order: tile t runs bfam_gpu_tile_elements elements per CTA
+ * with `threads` threads each (a tile with fewer threads than nodes or face
+ * nodes loops over them; each element of a CTA has its own shared-memory tile
+ * and barrier, down to one warp per element) and a register budget for
+ * `min_ctas` resident CTAs per SM.  Tile 0 is the single-domain kernel's (one
+ * element per CTA).  Every group of an order has as many tiles, but these
+ * shapes are those of the node-per-thread kernel (at 3D orders 6 and 7 the
+ * precision form's).  What a group runs under a tile depends on its precision
+ * and mesh too: bfam_gpu_tile_kernel. */
 int bfam_gpu_tile_count(int dim, int N);
 int bfam_gpu_tile_shape(int dim, int N, int tile, int *threads,
                         int *min_ctas);
 /* elements per CTA of tile t (>= 1), or a negative BFAM_GPU_E* code */
 int bfam_gpu_tile_elements(int dim, int N, int tile);
+/* The kernel of tile t in groups of one precision and kind of mesh (hanging:
+ * with hanging faces, see bfam_gpu_batch_group_mesh): its name -- "node", a
+ * thread per node; "pack", the nodes of several elements (tile 0 in 2D, but for
+ * the precision form at order 7, and at 3D orders 1 and 2); "mma", the FP64
+ * matrix instruction, a warp per plane of nodes (the plain form at 3D orders 6
+ * and 7 and, with hanging faces, 5) -- and per CTA its threads, the resident
+ * CTAs per SM of its register budget and its elements (at 3D order 2 "pack"
+ * groups below 48 elements per SM, 12 without hanging faces, run "node").  A
+ * group of one domain under tile 0 runs the single-domain form of tile 0. */
+int bfam_gpu_tile_kernel(int dim, int N, int precision, int hanging, int tile,
+                         char *name, size_t len, int *threads, int *min_ctas,
+                         int *elements);
 /* Choose group g's tile and the CTAs per SM its L2 lookahead assumes
  * (ctas_per_sm; 0: as many as fit). */
 int bfam_gpu_batch_set_tile(bfam_gpu_batch_t *b, int g, int tile,

@@ -80,3 +80,35 @@ def test_group_kinds():
     assert [(g["N"], g["domains"], g["hanging"]) for g in b.groups()] == \
         [(3, 2, False), (3, 1, True), (5, 1, True)]
     b.free()
+
+
+# kernels of the first tiles: what the dispatch runs
+FIRST = [(2, 4, 0, 0, "pack"), (2, 4, 1, 1, "pack"), (2, 7, 0, 0, "pack"), (2, 7, 1, 0, "node"),
+         (3, 1, 0, 1, "pack"), (3, 2, 1, 0, "pack"), (3, 3, 0, 1, "node"), (3, 4, 1, 1, "node"),
+         (3, 5, 0, 0, "node"), (3, 5, 0, 1, "mma"), (3, 5, 1, 1, "node"), (3, 6, 0, 0, "mma"),
+         (3, 6, 1, 1, "node"), (3, 7, 0, 1, "mma"), (3, 7, 1, 0, "node")]
+
+
+@pytest.mark.parametrize("dim,N,prec,hanging,kernel", FIRST)
+def test_tile_kernels(dim, N, prec, hanging, kernel):
+    t = bf.tile_kernels(dim, N, prec, bool(hanging))
+    assert t[0][0] == kernel
+    # as many as the order's shapes, and no two alike (the precision form's
+    # first budget at order 5 is also one of the others)
+    assert len(t) == len(bf.tile_shapes(dim, N))
+    assert len(set(t)) == len(t) - ((dim, N, prec) == (3, 5, 1))
+    for name, threads, minb, elements in t:
+        assert threads % 32 == 0 and threads <= 1024 and minb >= 1 and elements >= 1
+        assert name != "mma" or (threads == 32 * (N + 1) and elements == 1)
+
+
+def test_cache_key_names_the_kernels():
+    """a tile index is not reused for a group that runs other kernels under it"""
+    key = lambda *a, **k: autotune._key("GPU", *a, **k)
+    keys = {key(3, 5, 0, hanging=h, domains=d) for h in (False, True) for d in (1, 5)}
+    assert len(keys) == 4
+    assert key(3, 5, 0, domains=2) == key(3, 5, 0, domains=7)
+    assert "kernels:mma." in key(3, 5, 0, hanging=True)
+    assert "kernels:node." in key(3, 5, 0, hanging=False)
+    assert "kernels:pack." in key(2, 4, 0) and "kernels:pack." in key(3, 2, 1)
+    assert "kernels:mma." in key(3, 7, 0) and "kernels:node." in key(3, 7, 1)
