@@ -101,8 +101,23 @@ def measured_peak():
     return FALLBACK_HBM_GBS, "fallback"
 
 
+def group_kernel(choice):
+    """the kernel that a batch group runs under the tuner's choice"""
+    import bfam_b200 as bf
+    name = bf.tile_kernels(choice["dim"], choice["N"], choice["precision"],
+                           choice["hanging"])[choice["tile"]][0]
+    alone = choice["domains"] == 1 and choice["tile"] == 0 and choice["ctas_per_sm"] == 0
+    return f"dg_{'stage' if name == 'node' else name}_{'' if alone else 'batch_'}kernel"
+
+
+def stage_key(name, n, fp32, kernels):
+    """key of a captured stage: problem, base cells per axis, form and kernels"""
+    return "-".join([f"stage_{name}", f"n{n}", "fp32" if fp32 else "fp64",
+                     *sorted(set(kernels))])
+
+
 def profiled_traffic(kernel_key):
-    """dram bytes per launch from the committed ncu summary, if any."""
+    """dram bytes per LSRK stage from the committed ncu summary, if any."""
     f = ROOT / "profiles" / "traffic.txt"
     if not f.exists():
         return None
@@ -466,7 +481,8 @@ def run_batched(args):
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "peak_source": f"of {peak_kind}",
                          "traffic": None,
-                         "kernel": "dg_stage_batch_kernel (all order groups)"},
+                         "kernel": " + ".join(sorted({group_kernel(t) for t in tiles})) +
+                         " (all order groups)"},
             "plain_fp64_alone": {"value": plain_value, "unit": "DOF-updates/s",
                                  "instances": len(sample),
                                  "speedup_of_value": value / plain_value if plain_value else None,
@@ -860,11 +876,12 @@ def main():
     alg_bytes_per_stage = p.ndof * ALG_BYTES_PER_DOF_UPDATE[ns]
     achieved = alg_bytes_per_stage / per_stage_s / 1e9
     peak, peak_kind = measured_peak()
-    traffic = profiled_traffic(f"stage_{p.name}") if p.mesh.dim == 3 else None
+    kernels = dom.kernel_names()
+    traffic = profiled_traffic(stage_key(p.name, args.n, prec == bf.PRECISION_FP32, kernels))
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "peak_source": f"of {peak_kind}",
                 "traffic": traffic,
-                "kernel": ("dg_stage_kernel" if prec == bf.PRECISION_FP32 else "dg_mma_kernel") +
+                "kernel": " + ".join(sorted(set(kernels))) +
                 " (fused volume+face+mortar+LSRK update)",
                 "per": f"LSRK stage = {levels} launch(es), one per refinement level",
                 "alg_bytes_per_stage": alg_bytes_per_stage,

@@ -171,6 +171,7 @@ def _declare(L: C.CDLL) -> None:
         "bfam_gpu_pglue_free": (C.c_int, [vp]),
         "bfam_gpu_batch_add_pglue": (C.c_int, [vp, vp]),
         "bfam_gpu_batch_launches_per_step": (C.c_int, [vp]),
+        "bfam_gpu_domain_kernel_name": (C.c_int, [vp, C.c_int, C.c_char_p, C.c_size_t]),
         "bfam_gpu_domain_launch_levels": (C.c_int, [vp]),
         "bfam_gpu_batch_num_groups": (C.c_int, [vp]),
         "bfam_gpu_batch_group_info": (C.c_int, [vp, C.c_int, P(C.c_int), P(C.c_int),
@@ -532,6 +533,15 @@ class GpuDomain:
         if self.mesh is None:
             raise ValueError("the domain no longer holds its mesh")
         return write_vtu(path, self.mesh, self.get_fields(), time=time, binary=binary)
+
+    def kernel_names(self) -> list[str]:
+        """the kernel of each launch level's stages"""
+        out = []
+        for level in range(self.launch_levels()):
+            buf = C.create_string_buffer(64)
+            _check(lib().bfam_gpu_domain_kernel_name(self._h, level, buf, len(buf)))
+            out.append(buf.value.decode())
+        return out
 
     def launch_levels(self) -> int:
         """launches per LSRK stage (one per refinement level)"""

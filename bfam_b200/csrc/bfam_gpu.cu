@@ -1314,6 +1314,19 @@ int bfam_gpu_domain_launch_levels(const bfam_gpu_domain_t *d)
   return d ? d->nlevels : 0;
 }
 
+int bfam_gpu_domain_kernel_name(const bfam_gpu_domain_t *d, int level, char *buf,
+                                size_t len)
+{
+  if (!d || !buf || !len || level < 0 || level >= d->nlevels)
+    return fail(BFAM_GPU_EINVAL, "no launch level %d", level);
+  static const char *const name[] = {"dg_stage_kernel", "dg_pack_kernel",
+                                     "dg_mma_kernel"};
+  std::snprintf(buf, len, "%s",
+                name[d->ks.kernel(level_size(d, level), d->hops.data(), d->sms,
+                                  level_mode(d, level))]);
+  return 0;
+}
+
 int bfam_gpu_domain_free(bfam_gpu_domain_t *d)
 {
   release(d);

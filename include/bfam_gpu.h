@@ -306,6 +306,10 @@ int bfam_gpu_domain_sync(bfam_gpu_domain_t *dom);
  * with coarse-side hanging faces sums the projected mortar jumps that the
  * fine elements across those faces produce earlier in the same stage. */
 int bfam_gpu_domain_launch_levels(const bfam_gpu_domain_t *dom);
+/* Name of the kernel that the stages of launch level `level` run, as a profiler
+ * shows it. */
+int bfam_gpu_domain_kernel_name(const bfam_gpu_domain_t *dom, int level,
+                                char *buf, size_t len);
 
 /* ------------------------------------------------------------------------
  * Point source and receivers (the serving requests' solves).  No
