@@ -80,8 +80,8 @@ struct StageParams
   int first_stage; // A == 0: dq is not read
   int flux;        // 0 upwind, 1 central
   // one element per CTA: the CTA of work item i prefetches into L2 the
-  // element of item i + ahead (half a wave of resident CTAs later), so that
-  // its loads find L2 (0: no prefetch)
+  // element of item i + ahead (half a wave of resident CTAs later, a quarter in
+  // the matrix kernel at N = 7), so that its loads find L2 (0: no prefetch)
   int ahead;
   int sms;     // SMs of the device
   int widest = 0; // elements of the stage's largest launch
@@ -181,9 +181,10 @@ template <int DIM, int N> struct Shape
                                      : (DIM == 3 && N == 3) ? 12
                                                             : MINB;
   // dq read from global memory (L2) in the update instead of staged in
-  // shared memory: at 3D N=7 (two CTAs of 103 KB with dq staged leave the
-  // L1 cache about 22 KB for the neighbour-trace gathers; 105.6 vs 102.4 G
-  // DOF-updates/s in the plain form), and in the precision form at N=5
+  // shared memory, in the precision form (the plain form at N=7 is the matrix
+  // kernel's): at 3D N=7, where a CTA takes 85 KB so and 122 KB with dq staged,
+  // two of which an SM does not hold (one CTA 77.9, two 107.8 G
+  // DOF-updates/s), and at N=5, where staging was 9 % slower
   static constexpr bool DQ_L2 = DIM == 3 && N == 7;
   static constexpr bool DQ_L2_NARROW = DIM == 3 && N == 5;
   // Element rows of an odd number of nodes start on an 8-byte boundary in

@@ -86,7 +86,7 @@ __device__ __forceinline__ void for_arrays(int wid, int arrays,
 
 // The mode of a launch over a mesh without hanging faces: compiled without the
 // mortar passes (N = 3 157 -> 161 and 162 -> 166 G DOF-updates/s in the two
-// forms, N = 4 137 -> 140 and 154 -> 158, 2D N = 5 138 -> 143), but for two
+// forms, N = 4 137 -> 140 and 154 -> 158; the packed kernel's 2D N = 5 138 -> 143), but for two
 // shapes that ran slower so (the plain form at N = 5 spills: 158 against 162;
 // the precision form at 2D N = 7: 171 against 174)
 template <int DIM, int N, typename CT>
@@ -296,7 +296,7 @@ __device__ __forceinline__ void issue_element(const DomainView &d,
         bulk_g2s(dst + c * PITCH, src + c * fs + eoff - sh(c),
                  (PITCH - (last && c == NFLD - 1 ? 2 : 0)) * sizeof(double), bar);
     };
-    fence_proxy_async(); // shared memory of the previous element is free
+    fence_proxy_async(); // the copies complete on barriers set up just now
     // the face flux constants with the state, so that no thread needs
     // another thread's copies before the face phase
     rows(qs, d.qin, bar_q, 4 * NF);

@@ -36,8 +36,10 @@ extern std::atomic<uint64_t> g_prepares;
 // drain.  The kernel must call grid_dependency_wait in every CTA before it
 // touches anything an earlier kernel writes.  A step of a small mesh is a
 // chain of such latencies: 2D N = 4 on 16 x 16 elements 18.5 -> 16.4 us per
-// step of five launches replayed from a graph and 30.7 -> 15.4 us eagerly, 3D
-// N = 5 on 211 elements 71.7 -> 69.9 and 92.2 -> 66.1 us per ten launches.
+// step of five launches replayed from a graph, and eagerly 30.7 -> 15.4 where
+// the steps are waited for (13.6 -> 12.5 in a stream of steps, which the host's
+// launch calls bound), 3D N = 5 on 211 elements 71.7 -> 69.9 and 92.2 -> 66.1 us
+// per ten launches.
 // overlap false: an ordinary launch (kernels among others on other streams).
 template <typename... P, typename... A>
 cudaError_t launch_dependent(bool overlap, void (*kernel)(P...), dim3 grid,
@@ -58,22 +60,22 @@ cudaError_t launch_dependent(bool overlap, void (*kernel)(P...), dim3 grid,
 }
 
 // sp with StageParams::early for a stage whose widest launch has `ctas` CTAs
-// (LATE_FROM: see late_from).  A stage of less than a wave of CTAs leaves
+// (from: see late_from).  A stage of less than a wave of CTAs leaves
 // places free on its SMs.  If the next launch's CTAs take them early, the SMs
 // that finish first take more than their share of them, and the slowest SM of
 // the next launch, with one CTA more than it need have, sets its time.  So from
-// LATE_FROM of a wave (there is room for the next launch's CTAs beside them
+// `from` per cent of a wave (there is room for the next launch's CTAs beside them
 // below) to 85 % (hardly a place is free above), and not on meshes of at most a
 // CTA per SM, the next launch's CTAs wait for the end, and only its launch
 // overlaps it.  Us per step, ordinary launches -> early -> by this rule, replayed
 // from a graph: 3D N = 5 FP64, 440 conforming elements (0.59 of a wave)
-// 45.6 -> 50.8 -> 41.5, 528 49.7 -> 53.7 -> 47.7, 651 with hanging faces
-// 93.0 -> 96.2 -> 89.1; N = 4, 528 38.4 -> 43.5 -> 35.3; N = 6, 256
+// 45.6 -> 50.7 -> 42.1, 528 49.7 -> 53.6 -> 47.6, 651 with hanging faces
+// 93.0 -> 96.1 -> 90.2; N = 4, 528 38.4 -> 43.5 -> 35.3; N = 6, 256
 // 48.7 -> 59.9 -> 46.5; N = 2, 2,744 (0.58) 55.2 -> 60.7 -> 53.4.  Waiting always
 // costs small meshes 0.2 to 0.4 us a launch (2D N = 4, 256 16.9 -> 18.9).
-inline StageParams with_early(int ctas, StageParams sp, int late_from)
+inline StageParams with_early(int ctas, StageParams sp, int from)
 {
-  sp.early = ctas <= sp.sms || 100 * (int64_t)ctas <= late_from * (int64_t)sp.slots ||
+  sp.early = ctas <= sp.sms || 100 * (int64_t)ctas <= from * (int64_t)sp.slots ||
              100 * (int64_t)ctas >= 85 * (int64_t)sp.slots;
   return sp;
 }
