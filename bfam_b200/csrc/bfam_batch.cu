@@ -36,8 +36,9 @@ namespace
 typedef cudaError_t (*batch_launch_fn)(const DomainView *, const int2 *, int,
                                 const StageParams &, const double *hops,
                                 int grid, cudaStream_t, bool overlap);
-// for launches of n elements in one stage mode
-typedef cudaError_t (*batch_prepare_fn)(int mode, int n, int sms);
+// for launches of n elements in one stage mode, in a stage whose largest launch
+// has `widest`
+typedef cudaError_t (*batch_prepare_fn)(int mode, int n, int widest, int sms);
 typedef int (*batch_occupancy_fn)(int mode);
 
 struct BatchTile
@@ -114,7 +115,7 @@ struct TileImpl
            : mode == MODE_STAGE_NC ? kernel<MODE_STAGE_NC>
                                    : kernel<MODE_STAGE>;
   }
-  static cudaError_t prepare(int mode, int, int)
+  static cudaError_t prepare(int mode, int, int, int)
   {
     return allow_smem(of(mode), SMEM);
   }
@@ -141,18 +142,21 @@ struct TileImpl
 template <int DIM, int N, typename CT> struct PackTile
 {
   using K = PackShape<DIM, N, CT>;
-  using Small =
-      TileImpl<DIM, N, Shape<DIM, N>::NT, stage_min_ctas<DIM, N, CT>(), CT>;
+  // the node-per-thread kernel for small launches; at 3D N = 2 in the precision
+  // form 14 CTAs at 72 registers (5,077 refined elements 138 -> 132 us per step;
+  // alone ten are as fast or faster, 5,172 114 and 116)
+  using Small = TileImpl<DIM, N, Shape<DIM, N>::NT,
+                         DIM == 3 ? 14 : stage_min_ctas<DIM, N, CT>(), CT>;
   template <int MODE>
   static cudaError_t run(const DomainView *v, const int2 *w, int nwork,
                          const StageParams &sp, const double *hops, int,
                          cudaStream_t st, bool overlap)
   {
-    if constexpr (pack_has_small<DIM, N>())
+    if constexpr (pack_has_small<DIM, N, CT>(true))
     {
       constexpr int M =
           MODE == MODE_STAGE_CF ? conforming_mode<DIM, N, CT>() : MODE;
-      if (pack_too_small<DIM, N>(nwork, sp.sms, MODE))
+      if (pack_too_small<DIM, N, CT>(nwork, sp.widest, sp.sms, MODE, true))
         return Small::template run<M>(v, w, nwork, sp, hops, nwork, st,
                                       overlap);
     }
@@ -160,11 +164,7 @@ template <int DIM, int N, typename CT> struct PackTile
     const StageParams pp = pack_params<DIM, N, K::E>(nwork, sp);
     return launch_dependent(overlap, dg_pack_batch_kernel<DIM, N, MODE, CT>,
                             pack_ctas(nwork, pp), K::NT, K::BYTES, st, v, w,
-                            nwork,
-                            with_early(pack_ctas(sp.widest, pack_params<DIM, N, K::E>(
-                                                                sp.widest, sp)),
-                                       pp, pack_late_from<DIM, N, CT>()),
-                            dop);
+                            nwork, pp, dop);
   }
   static auto of(int mode)
   {
@@ -172,12 +172,12 @@ template <int DIM, int N, typename CT> struct PackTile
            : mode == MODE_STAGE_NC ? dg_pack_batch_kernel<DIM, N, MODE_STAGE_NC, CT>
                                    : dg_pack_batch_kernel<DIM, N, MODE_STAGE, CT>;
   }
-  static cudaError_t prepare(int mode, int n, int sms)
+  static cudaError_t prepare(int mode, int n, int widest, int sms)
   {
-    if constexpr (pack_has_small<DIM, N>())
+    if constexpr (pack_has_small<DIM, N, CT>(true))
     {
-      if (pack_too_small<DIM, N>(n, sms, mode))
-        return Small::prepare(mode, n, sms);
+      if (pack_too_small<DIM, N, CT>(n, widest, sms, mode, true))
+        return Small::prepare(mode, n, widest, sms);
     }
     return allow_smem(of(mode), K::BYTES);
   }
@@ -203,7 +203,7 @@ template <int DIM, int N, typename CT> struct PackTile
 // the first tile of a shape: the single-domain kernel's
 template <int DIM, int N, typename CT> BatchTile first_tile()
 {
-  if constexpr (use_pack<DIM, N, CT>())
+  if constexpr (use_pack_batch<DIM, N, CT>())
     return PackTile<DIM, N, CT>::make();
   else
     return TileImpl<DIM, N, Shape<DIM, N>::NT, stage_min_ctas<DIM, N, CT>(),
@@ -224,7 +224,7 @@ template <int N, int MINB> struct MmaTile
                             with_early(sp.widest, sp, MMA_LATE_FROM),
                             1.0 / hops[7 * (N + 1) * (N + 1)]);
   }
-  static cudaError_t prepare(int, int, int)
+  static cudaError_t prepare(int, int, int, int)
   {
     return allow_smem(kernel, M::BYTES);
   }
@@ -599,7 +599,7 @@ int choose_grid(bfam_gpu_batch_t *b, bfam_gpu_batch_t::Group &g)
   const BatchTile &t = g.tiles[g.tile];
   // the kernels that the group's levels launch
   for (size_t l = 0; l < g.work.size(); ++l)
-    CUDA_TRY(t.prepare(group_mode(g, l), (int)g.nwork_l[l], b->sms));
+    CUDA_TRY(t.prepare(group_mode(g, l), (int)g.nwork_l[l], g.widest, b->sms));
   int occ = t.occupancy(group_mode(g, 0));
   if (occ <= 0)
     return fail(BFAM_GPU_EUNSUPPORTED,

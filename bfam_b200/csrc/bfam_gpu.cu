@@ -102,9 +102,9 @@ int stage_kernel(int n, const double *hops, int sms, int mode)
     if (mesh_hangs(hops, N))
       return KERNEL_MMA;
   }
-  if constexpr (pack_has_small<DIM, N>())
+  if constexpr (pack_has_small<DIM, N, CT>(false))
   {
-    if (pack_too_small<DIM, N>(n, sms, mode))
+    if (pack_too_small<DIM, N, CT>(n, n, sms, mode, false))
       return KERNEL_NODE;
   }
   return use_mma<DIM, N, CT>()    ? KERNEL_MMA
@@ -130,9 +130,7 @@ cudaError_t pack_launch(const DomainView &v, int n, const StageParams &sp,
       : mode == MODE_STAGE_NC ? pack_kernel<DIM, N, CT, MODE_STAGE_NC>
       : mode == MODE_STAGE_CF ? pack_kernel<DIM, N, CT, MODE_STAGE_CF>
                               : pack_kernel<DIM, N, CT, MODE_RHS>,
-      pack_ctas(n, pp), K::NT, K::BYTES, stream, v, n,
-      with_early(pack_ctas(sp.widest, pack_params<DIM, N, K::E>(sp.widest, sp)), pp,
-                 pack_late_from<DIM, N, CT>()), dop);
+      pack_ctas(n, pp), K::NT, K::BYTES, stream, v, n, pp, dop);
 }
 
 // n work items, a CTA for each element (packed: for several)
@@ -153,7 +151,7 @@ cudaError_t stage_launch(const DomainView &v, int n, const StageParams &sp,
       return pack_launch<DIM, N, CT>(v, n, sp, hops, mode, stream, overlap);
   }
   if constexpr (!use_mma<DIM, N, CT>() &&
-                (!use_pack<DIM, N, CT>() || pack_has_small<DIM, N>()))
+                (!use_pack<DIM, N, CT>() || pack_has_small<DIM, N, CT>(false)))
     return node_launch<DIM, N, CT>(v, n, sp, hops, mode, stream, overlap);
   else
     return cudaErrorInvalidDeviceFunction;
@@ -198,7 +196,7 @@ cudaError_t stage_prepare(int k, int mode, int *occ)
           K::NT, K::BYTES, occ);
   }
   if constexpr (!use_mma<DIM, N, CT>() &&
-                (!use_pack<DIM, N, CT>() || pack_has_small<DIM, N>()))
+                (!use_pack<DIM, N, CT>() || pack_has_small<DIM, N, CT>(false)))
     return prepare_one(
         mode == MODE_STAGE      ? single_kernel<DIM, N, CT, MODE_STAGE>
         : mode == MODE_STAGE_NC ? single_kernel<DIM, N, CT, MODE_STAGE_NC>

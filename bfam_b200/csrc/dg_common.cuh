@@ -160,6 +160,9 @@ template <int DIM, int N> struct Shape
   //     (109.1-109.4 vs 105.1-105.3 with seven; 105.6 with twelve), twelve
   //     in the precision form, which then reads dq from L2 (115.4 vs 104.3
   //     with seven, 109.2 with ten);
+  //   3D N=2: 11 CTAs of 64 threads, at 80 registers, in the plain form (5,202
+  //     conforming elements 84.9 -> 77.1 us per step, 7,847 in a batch 137 ->
+  //     126; refined 8,211 189 -> 169), ten in the precision form;
   //   3D N=4: six CTAs of 160 threads in the plain form (137 conforming and
   //     106 refined; four 128 and 94, seven 132 and 100, eight 134 and 104),
   //     seven in the precision form (156 and 117; four 134 and 96, six 143
@@ -174,6 +177,7 @@ template <int DIM, int N> struct Shape
       : (DIM == 3 && N == 5) ? 5
       : (DIM == 3 && N == 4) ? 6
       : (DIM == 3 && N == 3) ? 10
+      : (DIM == 3 && N == 2) ? 11
                              : (MINB_RAW < 1 ? 1 : (MINB_RAW > 16 ? 16 : MINB_RAW));
   static constexpr int MINB_NARROW = (DIM == 3 && N == 5)   ? 4
                                      : (DIM == 3 && N == 4) ? 7

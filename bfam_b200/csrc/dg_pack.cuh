@@ -13,10 +13,10 @@
 // conforming and with 30 % of the base cells refined): 2D N = 1 28 -> 86 and
 // 22 -> 63, N = 2 48 -> 117 and 36 -> 81, N = 3 82 -> 143 and 56 -> 116, N = 4
 // 81 -> 143 and 68 -> 110, N = 5 91 -> 143 and 65 -> 112, N = 6 81 -> 126 and
-// 67 -> 97, N = 7 141 -> 150 and 103 -> 118, N = 8 90 -> 118 and 79 -> 95; 3D
-// N = 1 56 -> 96 and 38 -> 62, N = 2 80 -> 98 and 58 -> 72.  Not used where the
-// one-element kernel is faster: 3D N = 3 (156 against 123) and 4, and the
-// precision form at 2D N = 7 (173 against 162).
+// 67 -> 97, N = 7 141 -> 150 and 103 -> 118, N = 8 (precision form) 105 -> 135
+// and 89 -> 106; 3D N = 1 56 -> 96 and 38 -> 62, N = 2 80 -> 98 and 58 -> 72.  Not
+// used where the one-element kernel is faster: 3D N = 3 (156 against 123) and 4,
+// the shapes of use_pack, and launches too small for it (pack_from).
 // What bounds it now is latency (long scoreboard) beside the LSU pipe (60 %).
 #pragma once
 
@@ -58,11 +58,25 @@ template <int DIM, int N, typename CT> struct PackShape
   static constexpr int MINB = BY_SMEM < WANT ? BY_SMEM : WANT;
 };
 
-// shapes and arithmetic the kernel serves
+// Shapes and arithmetic the kernel serves.  Not, of 2D's, the precision form at
+// N = 7, and the plain form at N = 8, whose one element of 81 nodes per CTA,
+// its rows by bulk copies, is as fast on large meshes (74,000 elements 1,259 us
+// per step against 1,278 here, refined 1,562 and 1,583) and faster on small ones
+// (1,501 refined 60.5 and 70.7) and in batches (73,600 refined 1,699 and 1,798).
 template <int DIM, int N, typename CT>
 __host__ __device__ constexpr bool use_pack()
 {
-  return DIM == 2 ? N != 7 || sizeof(CT) == sizeof(double) : N <= 2;
+  return DIM == 2 ? N < 7 || N == (sizeof(CT) == sizeof(double) ? 7 : 8) : N <= 2;
+}
+
+// In batches of several domains not the plain form at 3D N = 2: the
+// node-per-thread kernel is faster or equal (5,256 conforming elements 91 us per
+// step against 112 here, 242,649 3,352 and 3,419; refined 39,335 826 and 847,
+// 248,268 4,781 and 4,733).
+template <int DIM, int N, typename CT> constexpr bool use_pack_batch()
+{
+  return use_pack<DIM, N, CT>() &&
+         !(DIM == 3 && N == 2 && sizeof(CT) == sizeof(double));
 }
 
 // Low orders, whose CTA holds many elements: on a small mesh a CTA takes only
@@ -94,29 +108,49 @@ inline int pack_ctas(int n, const StageParams &sp)
   return (n + sp.per - 1) / sp.per;
 }
 
-// Launches of a served shape that are too small for it: at 3D N = 2 a CTA's
-// four elements have up to 12 fine faces and its 128 threads go through their
-// lines in turns, so below 48 elements per SM the node-per-thread kernel's many
-// small CTAs are faster (us per step packed and not: 398 refined elements 53
-// and 48, 1,597 76 and 60, 6,425 157 and 145, the few coarse-sided elements of
-// 28,168 553 and 533); without hanging faces below 12 (512 elements 25.4 and
-// 23.4, 1,728 42 and 35 in the precision form, 4,096 69 and 71).
-template <int DIM, int N> constexpr bool pack_has_small()
+// Launches of a served shape that are too small for it: the passes over a CTA's
+// fine faces go on among few of its threads, and in batches each of its elements
+// reaches its domain through two tables, so on meshes of a few elements per SM
+// the node-per-thread kernel's many small CTAs are faster.  The elements per SM
+// below which a launch goes there (with hanging faces or without, in a batch of
+// several domains or not; in 2D those of the stage's widest launch, whose levels
+// then go together) lie where the sides meet; us per step node-per-thread and
+// packed:
+//   3D N = 2, FP64: 9,969 refined elements 206 and 207, 24,254 468 and 461;
+//     conforming 2,197 46 and 57, 42,875 566 and 578, 64,000 827 and 822;
+//   FP32: 1,597 refined 64 and 76; conforming 1,331 34 and 35, 2,197 49 and 48;
+//     batches 5,077 refined 132 and 138, 125,382 2,374 and 2,427, conforming
+//     5,256 91 and 100, 40,661 571 and 573, 82,620 1,132 and 1,121;
+//   2D N = 6, batches: FP64 5,198 refined 108 and 116, 7,805 154 and 142,
+//     conforming 990 29.5 and 33.5, 1,521 41 and 40; FP32 alike;
+//   2D N = 7, FP64, batches: 5,198 refined 105 and 117, 11,557 216 and 220,
+//     17,246 321 and 312, conforming 3,384 59 and 65, 47,099 578 and 584;
+//   2D N = 8, FP32, batches: 3,401 refined 103 and 110, 5,198 150 and 135,
+//     conforming 990 31.4 and 37.5, 1,521 45.8 and 45.0.
+template <int DIM, int N, typename CT>
+constexpr int pack_from(bool hanging, bool batch)
 {
-  return DIM == 3 && N == 2;
+  constexpr bool f64 = sizeof(CT) == sizeof(double);
+  constexpr int always = 1 << 20;
+  if (DIM == 3 && N == 2)
+    return batch ? (hanging ? always : 400)
+                 : (hanging ? 48 : f64 ? 400 : 12);
+  if (DIM == 3 || N < 6 || !batch)
+    return 0;
+  return N == 6   ? (hanging ? 32 : 10)
+         : N == 7 ? (hanging ? 60 : always)
+                  : (hanging ? 22 : 8);
 }
-template <int DIM, int N> bool pack_too_small(int n, int sms, int mode)
+template <int DIM, int N, typename CT> constexpr bool pack_has_small(bool batch)
 {
-  return pack_has_small<DIM, N>() && n < (mode == MODE_STAGE_CF ? 12 : 48) * sms;
+  return pack_from<DIM, N, CT>(true, batch) > 0;
 }
-
-// As late_from: the plain form's launches at 3D N = 2 are long enough to wait for
-// (2,744 conforming elements, 0.58 of a wave, 60.7 us per step early and 53.4
-// late; in the precision form 45.9 and 47.5), others not (3D N = 1, 1,000 16.8
-// and 17.8).
-template <int DIM, int N, typename CT> constexpr int pack_late_from()
+// n elements in a stage whose largest launch has `widest`
+template <int DIM, int N, typename CT>
+bool pack_too_small(int n, int widest, int sms, int mode, bool batch)
 {
-  return DIM == 3 && N == 2 && sizeof(CT) == sizeof(double) ? 50 : 85;
+  return (DIM == 2 ? widest : n) <
+         (int64_t)pack_from<DIM, N, CT>(mode != MODE_STAGE_CF, batch) * sms;
 }
 
 // The 1-D mortar pass of line_apply on `lines` faces of NC fields each (2D
@@ -436,8 +470,7 @@ __device__ __forceinline__ void pack_elements(const Item &item, int n,
     }
   }
   __syncthreads();
-  if (sp.early)
-    grid_launch_dependents(); // as in dg_stage.cuh, not earlier
+  grid_launch_dependents(); // as in dg_stage.cuh, not earlier
   if (!mine)
     return;
 

@@ -116,6 +116,18 @@ __host__ __device__ constexpr bool mma_mortars()
   return DIM == 3 && N >= 3 && sizeof(CT) < sizeof(double);
 }
 
+// Per cent of a wave of resident CTAs from which a stage does not let the next
+// launch's CTAs in before its end; 85: never (as in
+// the packed kernel).  The short launches of 2D and of 3D orders up to 3 lose more by waiting than they gain (N = 3, 1,338 elements
+// with hanging faces 63.5 -> 65.4 us per step, 2D N = 5, 1,600 22.6 -> 25.1).
+// The others' lines lie where the sides meet: N = 5 FP64 conforming 360 elements
+// (0.49) 39.5 early and 41.4 late, 400 (0.54) 48.2 and 42.0; N = 5 FP32 256 (0.43)
+// 33.5 and 29.2, 360 (0.61) 38.7 and 37.3.
+template <int DIM, int N, typename CT> constexpr int late_from()
+{
+  return DIM == 2 || N <= 3 ? 85 : sizeof(CT) < sizeof(double) ? 42 : 50;
+}
+
 // Node of thread t in the volume/update pass.  Nodes go in order (i
 // fastest), except in 3D when a k-plane holds between 32 and 64 nodes (N = 5,
 // 6): then warp w < Nq takes the first 32 nodes of plane w and the remaining
@@ -622,7 +634,7 @@ __device__ __forceinline__ void compute_element(const DomainView &d,
   // at the kernel's start instead, its waiting CTAs crowd onto the SMs that
   // drain first (N = 5 on 1,057 elements 133 us per step against 127, 129
   // without the overlap)
-  if (sp.early)
+  if (late_from<DIM, N, CT>() == 85 || sp.early)
     grid_launch_dependents();
   // ------------------------ phase 2: volume, face contributions and update
   constexpr bool DQS = stage_dqs<DIM, N, CT>();
@@ -818,18 +830,6 @@ struct BatchItems
     prefetch_l2(work + idx);
   }
 };
-
-// Per cent of a wave of resident CTAs from which a stage does not let the next
-// launch's CTAs in before its end; 85: never.  The short launches of 2D and of
-// 3D orders up to 3 lose more by waiting than they gain (N = 3, 1,338 elements
-// with hanging faces 63.5 -> 65.4 us per step, 2D N = 5, 1,600 22.6 -> 25.1).
-// The others' lines lie where the sides meet: N = 5 FP64 conforming 360 elements
-// (0.49) 39.5 early and 41.4 late, 400 (0.54) 48.2 and 42.0; N = 5 FP32 256 (0.43)
-// 33.5 and 29.2, 360 (0.61) 38.7 and 37.3.
-template <int DIM, int N, typename CT> constexpr int late_from()
-{
-  return DIM == 2 || N <= 3 ? 85 : sizeof(CT) < sizeof(double) ? 42 : 50;
-}
 
 // One domain: item idx is element idx, or the idx-th of the launch's
 // element list (meshes with hanging faces launch their elements by level).

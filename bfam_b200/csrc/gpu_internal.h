@@ -71,8 +71,8 @@ cudaError_t launch_dependent(bool overlap, void (*kernel)(P...), dim3 grid,
 // from a graph: 3D N = 5 FP64, 440 conforming elements (0.59 of a wave)
 // 45.6 -> 50.7 -> 42.1, 528 49.7 -> 53.6 -> 47.6, 651 with hanging faces
 // 93.0 -> 96.1 -> 90.2; N = 4, 528 38.4 -> 43.5 -> 35.3; N = 6, 256
-// 48.7 -> 59.9 -> 46.5; N = 2, 2,744 (0.58) 55.2 -> 60.7 -> 53.4.  Waiting always
-// costs small meshes 0.2 to 0.4 us a launch (2D N = 4, 256 16.9 -> 18.9).
+// 48.7 -> 59.9 -> 46.5.  Waiting always costs
+// small meshes 0.2 to 0.4 us a launch (2D N = 4, 256 16.9 -> 18.9).
 inline StageParams with_early(int ctas, StageParams sp, int from)
 {
   sp.early = ctas <= sp.sms || 100 * (int64_t)ctas <= from * (int64_t)sp.slots ||

@@ -450,11 +450,12 @@ int bfam_gpu_tile_elements(int dim, int N, int tile);
 /* The kernel of tile t in groups of one precision and kind of mesh (hanging:
  * with hanging faces, see bfam_gpu_batch_group_mesh): its name -- "node", a
  * thread per node; "pack", the nodes of several elements (tile 0 in 2D, but for
- * the precision form at order 7, and at 3D orders 1 and 2); "mma", the FP64
+ * the precision form at order 7 and the plain form at 8, at 3D order 1 and, in
+ * the precision form, 2); "mma", the FP64
  * matrix instruction, a warp per plane of nodes (the plain form at 3D orders 6
  * and 7 and, with hanging faces, 5) -- and per CTA its threads, the resident
- * CTAs per SM of its register budget and its elements (at 3D order 2 "pack"
- * groups below 48 elements per SM, 12 without hanging faces, run "node").  A
+ * CTAs per SM of its register budget and its elements (small groups at 2D orders 6 to 8 and 3D order 2 run
+ * "node" where "pack" is given).  A
  * group of one domain under tile 0 runs the single-domain form of tile 0. */
 int bfam_gpu_tile_kernel(int dim, int N, int precision, int hanging, int tile,
                          char *name, size_t len, int *threads, int *min_ctas,

@@ -2,7 +2,6 @@
  * CTAs for which a stage does not let the next launch's CTAs in before its end
  * (host code; no device needed). */
 #include "dg_mma.cuh"
-#include "dg_pack.cuh"
 #include "dg_stage.cuh"
 #include "gpu_internal.h"
 
@@ -35,8 +34,5 @@ int main()
   show("node-2d-7", 8, late_from<2, 7, float>());
   show("mma-5", 5, MMA_LATE_FROM);
   show("mma-7", 2, MMA_LATE_FROM);
-  show("pack-2-fp64", 8, pack_late_from<3, 2, double>());
-  show("pack-2-fp32", 8, pack_late_from<3, 2, float>());
-  show("pack-2d", 10, pack_late_from<2, 4, double>());
   return 0;
 }

@@ -83,8 +83,8 @@ def test_group_kinds():
 
 
 # kernels of the first tiles: what the dispatch runs
-FIRST = [(2, 4, 0, 0, "pack"), (2, 4, 1, 1, "pack"), (2, 7, 0, 0, "pack"), (2, 7, 1, 0, "node"),
-         (3, 1, 0, 1, "pack"), (3, 2, 1, 0, "pack"), (3, 3, 0, 1, "node"), (3, 4, 1, 1, "node"),
+FIRST = [(2, 4, 0, 0, "pack"), (2, 4, 1, 1, "pack"), (2, 7, 0, 0, "pack"), (2, 7, 1, 0, "node"), (2, 8, 0, 0, "node"), (2, 8, 1, 0, "pack"),
+         (3, 1, 0, 1, "pack"), (3, 2, 1, 0, "pack"), (3, 2, 0, 0, "node"), (3, 3, 0, 1, "node"), (3, 4, 1, 1, "node"),
          (3, 5, 0, 0, "node"), (3, 5, 0, 1, "mma"), (3, 5, 1, 1, "node"), (3, 6, 0, 0, "mma"),
          (3, 6, 1, 1, "node"), (3, 7, 0, 1, "mma"), (3, 7, 1, 0, "node")]
 

@@ -37,14 +37,16 @@ def test_group_kernels():
     assert b.group_kernel(dict(g, hanging=False)) == "dg_stage_batch_kernel"
     assert b.group_kernel(dict(g, domains=1, tile=0)) == "dg_mma_kernel"
     assert b.group_kernel(dict(g, precision=1, domains=1, tile=0)) == "dg_stage_kernel"
-    assert b.group_kernel(dict(g, N=2, tile=0)) == "dg_pack_batch_kernel"
+    assert b.group_kernel(dict(g, N=2, tile=0, precision=1)) == "dg_pack_batch_kernel"
 
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("dim,N,n,p,prec,names", [
     (2, 4, (4, 4), 0.0, 0, ["pack"]), (2, 7, (4, 4), 0.0, 1, ["stage"]),
     (3, 1, (3, 3, 3), 0.4, 0, ["pack", "pack"]), (3, 2, (3, 3, 3), 0.4, 0, ["stage", "stage"]),
-    (3, 2, (13, 12, 12), 0.0, 0, ["pack"]), (3, 2, (16, 14, 15), 0.3, 0, ["pack", "stage"]),
+    (3, 2, (40, 39, 39), 0.0, 0, ["pack"]), (3, 2, (13, 12, 12), 0.0, 1, ["pack"]),
+    (3, 2, (13, 12, 12), 0.0, 0, ["stage"]), (2, 8, (4, 4), 0.4, 0, ["stage", "stage"]),
+    (2, 6, (4, 4), 0.4, 0, ["pack", "pack"]), (3, 2, (16, 14, 15), 0.3, 0, ["pack", "stage"]),
     (3, 3, (3, 3, 3), 0.4, 0, ["stage"] * 2), (3, 5, (2, 2, 2), 0.5, 0, ["mma"] * 2),
     (3, 5, (2, 2, 2), 0.0, 0, ["stage"]), (3, 5, (2, 2, 2), 0.5, 1, ["stage"] * 2),
     (3, 6, (2, 2, 2), 0.0, 0, ["mma"]), (3, 7, (2, 2, 2), 0.5, 0, ["mma"] * 2),

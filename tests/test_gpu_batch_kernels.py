@@ -92,28 +92,30 @@ def test_high_orders_under_every_tile(N, prec, tol, meshes):
         assert relerr(q, _oracle(prob, 3, source=True)).max() < tol
 
 
-# three uneven domains of one group, whose CTAs (with more than one element,
-# above 4 x 148 elements at orders 1 and 2) straddle their ends
-STRADDLE = [(2, 1, [((29, 23), 0.3), ((31, 17), 0.4), ((7, 5), 0.5)]),
-            (2, 2, [((27, 23), 0.4), ((19, 31), 0.3), ((3, 5), 0.4)]),
-            (2, 3, [((5, 3), 0.4), ((4, 7), 0.5), ((3, 3), 0.4)]),
-            (2, 6, [((3, 5), 0.4), ((7, 3), 0.5), ((2, 3), 0.4)]),
-            (2, 8, [((3, 3), 0.4), ((5, 3), 0.5), ((3, 4), 0.4)]),
-            (3, 1, [((8, 7, 7), 0.4), ((7, 5, 6), 0.3), ((3, 2, 3), 0.4)]),
-            (3, 2, [((13, 12, 13), 0.3), ((14, 13, 12), 0.3), ((3, 3, 2), 0.4)]),
-            (3, 2, [((11, 9, 7), 0.0), ((13, 9, 10), 0.0), ((3, 5, 1), 0.0)])]
+# three uneven domains of one group, whose CTAs straddle their ends: enough
+# elements that a CTA takes more than one (orders 1 and 2) and that the launch is
+# not left to the node-per-thread kernel (elements per SM: the last number)
+F64, F32 = PREC
+STRADDLE = [(2, 1, [((29, 23), 0.3), ((31, 17), 0.4), ((7, 5), 0.5)], PREC, 8),
+            (2, 2, [((27, 23), 0.4), ((19, 31), 0.3), ((3, 5), 0.4)], PREC, 8),
+            (2, 3, [((5, 3), 0.4), ((4, 7), 0.5), ((3, 3), 0.4)], PREC, 0),
+            (2, 6, [((59, 53), 0.4), ((7, 3), 0.5), ((13, 13), 0.4)], PREC, 32),
+            (2, 7, [((83, 79), 0.4), ((7, 3), 0.5), ((13, 13), 0.4)], [F64], 60),
+            (2, 8, [((43, 47), 0.4), ((5, 3), 0.5), ((11, 13), 0.4)], [F32], 22),
+            (2, 6, [((37, 41), 0.0), ((7, 3), 0.0), ((5, 5), 0.0)], PREC, 10),
+            (3, 1, [((8, 7, 7), 0.4), ((7, 5, 6), 0.3), ((3, 2, 3), 0.4)], PREC, 8),
+            (3, 2, [((39, 37, 41), 0.0), ((13, 9, 10), 0.0), ((3, 5, 1), 0.0)], [F32], 400)]
 
 
-@pytest.mark.parametrize("dim,N,meshes", STRADDLE, ids=str)
-@pytest.mark.parametrize("prec,tol", PREC, ids=IDS)
-def test_different_domains_inside_a_cta(dim, N, meshes, prec, tol):
+@pytest.mark.parametrize("dim,N,meshes,prec,tol,per_sm",
+                         [c[:3] + pt + c[4:] for c in STRADDLE for pt in c[3]], ids=str)
+def test_different_domains_inside_a_cta(dim, N, meshes, prec, tol, per_sm):
     probs = [_problem(dim, N, n, p, 7 + k, bounded=k == 1) for k, (n, p) in enumerate(meshes)]
     hanging = meshes[0][1] > 0
     kernel, _, _, per = bf.tile_kernels(dim, N, prec, hanging)[0]
     assert kernel == "pack" and per > 1
-    K = sum(p[0].K for p in probs)
-    assert N > 2 or K > 4 * 148 * 2
-    assert (dim, N) != (3, 2) or K > (72 if hanging else 12) * 148
+    # of a mesh with hanging faces at least 0.7 are in the first launch
+    assert (0.7 if hanging else 1.0) * sum(p[0].K for p in probs) > per_sm * 148
     alone = _alone(probs, prec, 2)
     for (q, _), prob in zip(alone, probs):
         assert relerr(q, _oracle(prob, 2)).max() < tol
@@ -128,12 +130,13 @@ def test_different_domains_inside_a_cta(dim, N, meshes, prec, tol):
 
 # one mesh per shape above the sizes below which other kernels or one element
 # per CTA serve it: right-hand side, boundary faces, hanging faces, point source
-LARGE = [(2, 1, (29, 27), 0.4), (2, 2, (31, 23), 0.4), (3, 1, (9, 8, 8), 0.4),
-         (3, 2, (13, 12, 12), 0.0), (3, 2, (16, 14, 15), 0.35)]
+LARGE = [(2, 1, (29, 27), 0.4, PREC), (2, 2, (31, 23), 0.4, PREC), (2, 6, (47, 43), 0.4, PREC),
+         (2, 7, (53, 51), 0.4, [F64]), (2, 8, (47, 43), 0.4, [F32]), (3, 1, (9, 8, 8), 0.4, PREC),
+         (3, 2, (40, 39, 39), 0.0, [F64]), (3, 2, (13, 12, 12), 0.0, [F32]),
+         (3, 2, (16, 14, 15), 0.35, PREC)]
 
 
-@pytest.mark.parametrize("dim,N,n,p", LARGE, ids=str)
-@pytest.mark.parametrize("prec,tol", PREC, ids=IDS)
+@pytest.mark.parametrize("dim,N,n,p,prec,tol", [c[:4] + pt for c in LARGE for pt in c[4]], ids=str)
 def test_packed_kernel_on_large_meshes(dim, N, n, p, prec, tol):
     prob = _problem(dim, N, n, p, 2, bounded=True)
     m, rho, lam, mu, q, dt = prob
