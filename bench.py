@@ -618,7 +618,7 @@ def run_serving(args):
     # tile choices for the request orders, one request alone and several,
     # before any clock starts
     for N, count in ((3, 1), (3, 2), (5, 1), (5, 2)):
-        m = bf.Mesh(3, N, (8, 8, 8))
+        m = bf.Mesh(3, N, (16, 16, 16))
         ds = [bf.GpuDomain(m, 1.0, 2.0, 1.0, precision=prec, device=local)
               for _ in range(count)]
         b = bf.Batch(ds)

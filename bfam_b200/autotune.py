@@ -88,6 +88,7 @@ def tune_group(dim: int, N: int, precision: int, elements: int, steps: int = 4,
     stream = torch.cuda.Stream(device=device)
     b = Batch(doms)
     b.set_stream(stream.cuda_stream)
+    b.step(dts, 4)  # the device awake, the post-step kernel loaded
     table = []
     for tile, (kernel, threads, minb, epc) in enumerate(
             tile_kernels(dim, N, precision, hanging)):
@@ -96,7 +97,7 @@ def tune_group(dim: int, N: int, precision: int, elements: int, steps: int = 4,
                 b.set_tile(0, tile, cps)
             except BfamGpuError:
                 continue  # does not fit an SM on this device
-            b.step(dts, 1)  # capture + warm-up
+            b.step(dts, 2)  # capture (a graph per state parity) and warm-up
             e0 = torch.cuda.Event(enable_timing=True)
             e1 = torch.cuda.Event(enable_timing=True)
             e0.record(stream)

@@ -71,6 +71,21 @@ def test_the_tuned_batch_is_of_the_groups_kind(monkeypatch, hanging, domains):
 
 
 @pytest.mark.gpu
+def test_no_capture_is_timed(monkeypatch):
+    """a step is captured once per state parity; both are before the timed steps"""
+    calls, tiles = [], []
+    step, set_tile = bf.Batch.step, bf.Batch.set_tile
+    monkeypatch.setattr(bf.Batch, "step", lambda self, dt, n=1, **k: (
+        calls.append((len(tiles), n)), step(self, dt, n, **k))[1])
+    monkeypatch.setattr(bf.Batch, "set_tile", lambda self, *a: (
+        tiles.append(a), set_tile(self, *a))[1])
+    t = autotune.tune_group(3, 4, bf.PRECISION_FP64, 100, steps=3, domains=2)
+    assert len(t["table"]) == len(tiles)
+    for k in range(1, len(tiles) + 1):
+        assert [n for c, n in calls if c == k] == [2, 3]
+
+
+@pytest.mark.gpu
 def test_group_kinds():
     def dom(N, p):
         m = bf.Mesh(3, N, (2, 2, 2), refine_prob=p, seed=2)
