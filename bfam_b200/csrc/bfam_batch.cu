@@ -221,7 +221,7 @@ template <int N, int MINB> struct MmaTile
                      cudaStream_t st, bool overlap)
   {
     return launch_dependent(overlap, kernel, grid, M::NT, M::BYTES, st, v, w, nwork,
-                            with_early(sp.widest, sp, MMA_LATE_FROM),
+                            with_early(sp.widest, sp, mma_late_from<N>()),
                             1.0 / hops[7 * (N + 1) * (N + 1)]);
   }
   static cudaError_t prepare(int, int, int, int)

@@ -70,7 +70,7 @@ cudaError_t mma_launch(const DomainView &v, int n, const StageParams &sp,
   return launch_dependent(overlap,
                           mode == MODE_RHS ? mma_kernel<N, MODE_RHS>
                                            : mma_kernel<N, MODE_STAGE>,
-                          n, M::NT, M::BYTES, stream, v, n, with_early(sp.widest, sp, MMA_LATE_FROM),
+                          n, M::NT, M::BYTES, stream, v, n, with_early(sp.widest, sp, mma_late_from<N>()),
                           1.0 / hops[7 * (N + 1) * (N + 1)]);
 }
 

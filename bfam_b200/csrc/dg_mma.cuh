@@ -91,8 +91,12 @@ __host__ __device__ constexpr bool use_mma_hanging()
 }
 // as late_from: N = 5, 331 elements with hanging faces (262 of them, 0.35, in the
 // first launch) 76.2 us per step early and 72.3 late, 204 69.1 and 71.3; N = 6,
-// 256 (0.58) 59.9 and 46.6
-constexpr int MMA_LATE_FROM = 34;
+// 204 (160, 0.36) 83.4 and 89.6 in eager steps, 256 conforming (0.58) 59.9 and
+// 46.6; N = 7, 204 (0.54) 67.5 and 71.3, 256 conforming 41.9 and 41.5
+template <int N> constexpr int mma_late_from()
+{
+  return N == 5 ? 34 : N == 6 ? 42 : 85;
+}
 
 // hops: an order-N domain's operators Dr | interpolation[3] | projection[3] | w;
 // a domain without a glue grid, so without hanging faces, has identities for

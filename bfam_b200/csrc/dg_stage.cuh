@@ -119,13 +119,15 @@ __host__ __device__ constexpr bool mma_mortars()
 // Per cent of a wave of resident CTAs from which a stage does not let the next
 // launch's CTAs in before its end; 85: never (as in
 // the packed kernel).  The short launches of 2D and of 3D orders up to 3 lose more by waiting than they gain (N = 3, 1,338 elements
-// with hanging faces 63.5 -> 65.4 us per step, 2D N = 5, 1,600 22.6 -> 25.1).
+// with hanging faces 63.5 -> 65.4 us per step, 2D N = 5, 1,600 22.6 -> 25.1), and
+// at N = 7 in the precision form two CTAs per SM leave little to gain (204 with
+// hanging faces 96.3 -> 98.9).
 // The others' lines lie where the sides meet: N = 5 FP64 conforming 360 elements
 // (0.49) 39.5 early and 41.4 late, 400 (0.54) 48.2 and 42.0; N = 5 FP32 256 (0.43)
 // 33.5 and 29.2, 360 (0.61) 38.7 and 37.3.
 template <int DIM, int N, typename CT> constexpr int late_from()
 {
-  return DIM == 2 || N <= 3 ? 85 : sizeof(CT) < sizeof(double) ? 42 : 50;
+  return DIM == 2 || N <= 3 || N == 7 ? 85 : sizeof(CT) < sizeof(double) ? 42 : 50;
 }
 
 // Node of thread t in the volume/update pass.  Nodes go in order (i

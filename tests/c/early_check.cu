@@ -32,7 +32,9 @@ int main()
   show("node-5-fp64", 5, late_from<3, 5, double>());
   show("node-5-fp32", 4, late_from<3, 5, float>());
   show("node-2d-7", 8, late_from<2, 7, float>());
-  show("mma-5", 5, MMA_LATE_FROM);
-  show("mma-7", 2, MMA_LATE_FROM);
+  show("mma-5", 5, mma_late_from<5>());
+  show("mma-6", 3, mma_late_from<6>());
+  show("mma-7", 2, mma_late_from<7>());
+  show("node-7-fp32", 2, late_from<3, 7, float>());
   return 0;
 }

@@ -29,7 +29,8 @@ def test_ranges(tmp_path):
                           text=True).stdout.splitlines()}
     # per cent of a wave from which the next launch waits; none: never
     want = {"node-3-fp64": None, "node-4-fp64": 50, "node-5-fp64": 50, "node-5-fp32": 42,
-            "node-2d-7": None, "mma-5": 34, "mma-7": 34}
+            "node-2d-7": None, "mma-5": 34, "mma-6": 42, "mma-7": None,
+            "node-7-fp32": None}
     assert set(out) == set(want)
     for name, lo in want.items():
         slots, first, last, holes = out[name]
@@ -48,7 +49,7 @@ def test_ranges(tmp_path):
                                         (5, (6, 5, 4), 0.4, bf.PRECISION_FP64),
                                         (5, (7, 6, 6), 0.0, bf.PRECISION_FP32),
                                         (6, (7, 6, 6), 0.0, bf.PRECISION_FP64),
-                                        (7, (6, 6, 5), 0.0, bf.PRECISION_FP64)])
+                                        (6, (4, 4, 4), 0.5, bf.PRECISION_FP64)])
 def test_same_bits(N, n, p, prec):
     m = bf.Mesh(3, N, n, refine_prob=p, seed=1)
     rho, lam, mu = bf.material_random(m.K, 2)
