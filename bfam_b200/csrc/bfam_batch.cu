@@ -673,7 +673,6 @@ cudaError_t launch_post_step(bfam_gpu_batch_t *b, int p)
 int launch_level(bfam_gpu_batch_t *b, bfam_gpu_batch::Group &g, size_t l,
                  int par, const StageParams &sp, cudaStream_t st, bool overlap)
 {
-  const int mode = group_mode(g, l);
   if (alone(g))
   {
     const int i = g.doms[0];
@@ -682,10 +681,10 @@ int launch_level(bfam_gpu_batch_t *b, bfam_gpu_batch::Group &g, size_t l,
     v.dt = b->dt[i];
     if (d->nlevels > 1)
       v.elist = d->elist + d->level_off[l];
-    return launch_elements(d, v, (int)g.nwork_l[l], sp, mode, st, overlap);
+    return launch_planned(d, v, d->stage_plan[l], sp, st, overlap);
   }
   const BatchTile &t = g.tiles[g.tile];
-  CUDA_TRY(t.of(mode)(g.views[par], g.work[l], (int)g.nwork_l[l], sp,
+  CUDA_TRY(t.of(group_mode(g, l))(g.views[par], g.work[l], (int)g.nwork_l[l], sp,
                       g.hops.data(), g.grid[l], st, overlap));
   return 0;
 }

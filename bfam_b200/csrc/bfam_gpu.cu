@@ -133,13 +133,12 @@ cudaError_t pack_launch(const DomainView &v, int n, const StageParams &sp,
       pack_ctas(n, pp), K::NT, K::BYTES, stream, v, n, pp, dop);
 }
 
-// n work items, a CTA for each element (packed: for several)
+// n work items in kernel k, a CTA for each element (packed: for several)
 template <int DIM, int N, typename CT>
 cudaError_t stage_launch(const DomainView &v, int n, const StageParams &sp,
-                         const double *hops, int mode, cudaStream_t stream,
-                         bool overlap)
+                         const double *hops, int mode, int k,
+                         cudaStream_t stream, bool overlap)
 {
-  const int k = stage_kernel<DIM, N, CT>(n, hops, sp.sms, mode);
   if constexpr (use_mma<DIM, N, CT>() || use_mma_hanging<DIM, N, CT>())
   {
     if (k == KERNEL_MMA)
@@ -465,28 +464,59 @@ int level_mode(const bfam_gpu_domain_t *d, int l)
                             : MODE_STAGE_NC;
 }
 
-// Set-up of the kernel that serves a launch of n elements in a mode, once per
-// domain; which kernel it is in *k.
-cudaError_t prepare_launch(bfam_gpu_domain_t *d, int n, int mode, int *k)
+// The launch of n elements in a mode: which kernel serves it, set up once per
+// domain, and what follows from its resident CTAs.
+cudaError_t plan_launch(bfam_gpu_domain_t *d, int n, int mode, LaunchPlan *p)
 {
-  *k = d->ks.kernel(n, d->hops.data(), d->sms, mode);
-  int &occ = d->ks.occ[*k][mode];
-  if (occ)
-    return cudaSuccess;
-  const cudaError_t e = d->ks.prepare(*k, mode, &occ);
-  return e == cudaSuccess && occ < 1 ? cudaErrorInvalidConfiguration : e;
-}
-
-int launch_elements(bfam_gpu_domain_t *d, const DomainView &v, int n,
-                    StageParams sp, int mode, cudaStream_t stream, bool overlap)
-{
-  int k;
-  CUDA_TRY(prepare_launch(d, n, mode, &k));
+  p->n = n;
+  p->mode = mode;
+  p->kernel = d->ks.kernel(n, d->hops.data(), d->sms, mode);
+  int &occ = d->ks.occ[p->kernel][mode];
+  if (!occ)
+  {
+    const cudaError_t e = d->ks.prepare(p->kernel, mode, &occ);
+    if (e != cudaSuccess || occ < 1)
+    {
+      occ = 0;
+      return e != cudaSuccess ? e : cudaErrorInvalidConfiguration;
+    }
+  }
+  p->slots = occ * d->sms;
   // prefetch part of a wave of resident CTAs ahead (half a wave: about half a
   // CTA lifetime before the element's CTA starts)
-  sp.slots = d->ks.occ[k][mode] * d->sms;
-  sp.ahead = sp.slots * (k == KERNEL_PACK ? d->ks.elements : 1) / d->ks.lookahead;
-  CUDA_TRY(d->ks.launch(v, n, sp, d->hops.data(), mode, stream, overlap));
+  p->ahead = p->slots * (p->kernel == KERNEL_PACK ? d->ks.elements : 1) /
+             d->ks.lookahead;
+  return cudaSuccess;
+}
+
+// the launches of a stage (rhs: of a right-hand side), one per level
+cudaError_t plan_levels(bfam_gpu_domain_t *d, bool rhs,
+                        std::vector<LaunchPlan> *plans)
+{
+  plans->assign(d->nlevels, LaunchPlan());
+  for (int l = 0; l < d->nlevels; ++l)
+  {
+    const cudaError_t e = plan_launch(
+        d, level_size(d, l), rhs ? MODE_RHS : level_mode(d, l), &(*plans)[l]);
+    if (e != cudaSuccess)
+    {
+      plans->clear();
+      return e;
+    }
+  }
+  return cudaSuccess;
+}
+
+int launch_planned(bfam_gpu_domain_t *d, const DomainView &v,
+                   const LaunchPlan &p, StageParams sp, cudaStream_t stream,
+                   bool overlap)
+{
+  sp.sms = d->sms;
+  sp.widest = d->widest;
+  sp.slots = p.slots;
+  sp.ahead = p.ahead;
+  CUDA_TRY(d->ks.launch(v, p.n, sp, d->hops.data(), p.mode, p.kernel, stream,
+                        overlap));
   return 0;
 }
 
@@ -500,20 +530,19 @@ int launch_stage(bfam_gpu_domain_t *d, int in, double A, double B, double C,
   sp.C = C;
   sp.first_stage = first;
   sp.flux = d->flux;
-  sp.sms = d->sms;
-  for (int l = 0; l < d->nlevels; ++l)
-    sp.widest = std::max(sp.widest, level_size(d, l));
+  std::vector<LaunchPlan> &plans = mode == MODE_RHS ? d->rhs_plan : d->stage_plan;
+  if (plans.empty())
+    CUDA_TRY(plan_levels(d, mode == MODE_RHS, &plans));
   DomainView v = view(d, in);
   v.dt = dt;
   // one launch per level; level l's elements after level l-1's
   for (int l = 0; l < d->nlevels; ++l)
   {
-    const int n = level_size(d, l);
+    const int n = plans[l].n;
     if (d->nlevels > 1)
       v.elist = d->elist + d->level_off[l];
     if (n == 0)
       continue;
-    const int m = mode == MODE_STAGE ? level_mode(d, l) : mode;
     bfam_gpu_domain::ProfLaunch pl{};
     if (d->prof)
     {
@@ -538,7 +567,7 @@ int launch_stage(bfam_gpu_domain_t *d, int in, double A, double B, double C,
     // overlapped also where a program steps several domains on their own
     // streams: 4 domains of 118 refined elements at N = 3 58.7 us per step of
     // all without and 49.1 with, of 692 at N = 5 233 and 227
-    if (int rc = launch_elements(d, v, n, sp, m, d->stream, true))
+    if (int rc = launch_planned(d, v, plans[l], sp, d->stream, true))
       return rc;
     g_launches.fetch_add(1, std::memory_order_relaxed);
     if (d->prof)
@@ -1204,11 +1233,10 @@ static int create_domain(const bfam_gpu_volume_t *vol,
     // alone: at its first call); set-up loads a kernel, 0.05 ms each (the
     // first conforming domain of 3D order 2 1.5 ms with all eight of its
     // shape's kernels, 1.0 with the one that it launches)
-    for (int l = 0; l < d->nlevels && ce == cudaSuccess; ++l)
-    {
-      int k;
-      ce = prepare_launch(d, level_size(d, l), level_mode(d, l), &k);
-    }
+    for (int l = 0; l < d->nlevels; ++l)
+      d->widest = std::max(d->widest, level_size(d, l));
+    if (ce == cudaSuccess)
+      ce = plan_levels(d, false, &d->stage_plan);
     if (ce != cudaSuccess)
     {
       release(d);
@@ -1319,9 +1347,7 @@ int bfam_gpu_domain_kernel_name(const bfam_gpu_domain_t *d, int level, char *buf
     return fail(BFAM_GPU_EINVAL, "no launch level %d", level);
   static const char *const name[] = {"dg_stage_kernel", "dg_pack_kernel",
                                      "dg_mma_kernel"};
-  std::snprintf(buf, len, "%s",
-                name[d->ks.kernel(level_size(d, level), d->hops.data(), d->sms,
-                                  level_mode(d, level))]);
+  std::snprintf(buf, len, "%s", name[d->stage_plan[level].kernel]);
   return 0;
 }
 

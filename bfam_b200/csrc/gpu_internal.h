@@ -94,7 +94,8 @@ enum
 // opt-in, resident CTAs per SM
 typedef cudaError_t (*stage_launch_fn)(const DomainView &, int n,
                                 const StageParams &, const double *D,
-                                int mode, cudaStream_t, bool overlap);
+                                int mode, int kernel, cudaStream_t,
+                                bool overlap);
 typedef int (*stage_kernel_fn)(int n, const double *hops, int sms, int mode);
 typedef cudaError_t (*prepare_fn)(int kernel, int mode, int *occ);
 typedef void (*energy_fn)(const double *, size_t, const ElemData *,
@@ -110,6 +111,13 @@ struct KernelSet
   int occ[3][4] = {}; // resident CTAs per SM by kernel and mode (0: not set up)
   int elements = 1;   // elements per CTA of the packed kernel
   int lookahead = 2;  // L2 lookahead: that part of a wave of resident CTAs
+};
+
+// a launch of a domain's stages: elements, mode, kernel, its resident CTAs on the
+// device and its L2 lookahead
+struct LaunchPlan
+{
+  int n = 0, mode = 0, kernel = 0, slots = 0, ahead = 0;
 };
 
 // the kernels of one (dim, order, precision)
@@ -142,6 +150,9 @@ struct bfam_gpu_domain
   int flux = 0, precision = 0;
   size_t fs = 0;
   bfam_b200::host::KernelSet ks;
+  // per launch level; of the right-hand side once it is called
+  std::vector<bfam_b200::host::LaunchPlan> stage_plan, rhs_plan;
+  int widest = 0; // elements of the largest level
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   double *q[2] = {nullptr, nullptr};
@@ -247,9 +258,10 @@ int upload(bfam_gpu_domain_t *d, T **dst, const T *src, size_t n)
 
 // the stage kernel's view of a domain whose stage input is q[in]
 DomainView view(bfam_gpu_domain_t *d, int in);
-// one launch over n elements of v, the domain's view
-int launch_elements(bfam_gpu_domain_t *d, const DomainView &v, int n,
-                    StageParams sp, int mode, cudaStream_t stream, bool overlap);
+// one launch of a plan over v, the domain's view
+int launch_planned(bfam_gpu_domain_t *d, const DomainView &v,
+                   const LaunchPlan &p, StageParams sp, cudaStream_t stream,
+                   bool overlap);
 int launch_stage(bfam_gpu_domain_t *d, int in, double A, double B, double C,
                  double dt, int first, int mode);
 
