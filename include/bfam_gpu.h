@@ -451,12 +451,12 @@ int bfam_gpu_tile_elements(int dim, int N, int tile);
  * with hanging faces, see bfam_gpu_batch_group_mesh): its name -- "node", a
  * thread per node; "pack", the nodes of several elements (tile 0 in 2D, but for
  * the precision form at order 7 and the plain form at 8, at 3D order 1 and, in
- * the precision form, 2); "mma", the FP64
- * matrix instruction, a warp per plane of nodes (the plain form at 3D orders 6
- * and 7 and, with hanging faces, 5) -- and per CTA its threads, the resident
- * CTAs per SM of its register budget and its elements (small groups at 2D orders 6 to 8 and 3D order 2 run
- * "node" where "pack" is given).  A
- * group of one domain under tile 0 runs the single-domain form of tile 0. */
+ * the precision form, 2; small groups at 2D orders 6 to 8 and 3D order 2 run
+ * "node" instead); "mma", the FP64 matrix instruction, a warp per plane of nodes
+ * (the plain form at 3D orders 6 and 7 and, with hanging faces, 5) -- and per
+ * CTA its threads, the resident CTAs per SM of its register budget and its
+ * elements.  A group of one domain under tile 0 runs its domain's own kernel
+ * (bfam_gpu_domain_kernel_name). */
 int bfam_gpu_tile_kernel(int dim, int N, int precision, int hanging, int tile,
                          char *name, size_t len, int *threads, int *min_ctas,
                          int *elements);
